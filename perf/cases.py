@@ -12,6 +12,7 @@ from __future__ import annotations
 
 import math
 
+import numpy as np
 import torch
 
 import adaptq_b200
@@ -127,59 +128,60 @@ def _fill(append, tokens, lead, dim, dist, gen):
     return scale
 
 
-def prepare(case, seed):
-    c = dict(case)
+def _draw_inputs(case, seed, append):
+    """Everything a case is given, in one order: the tokens already in the cache go to `append`
+    as (tokens, ..., dim) chunks; the token, prompt and queries of the pass come back."""
+    c, kind, dist, dim = case, case["kind"], case["dist"], case["dim"]
     gen = torch.Generator(device="cuda").manual_seed(int(seed) & (2**63 - 1))
-    kind, dist, dim = c["kind"], c["dist"], c["dim"]
-    s = {"kind": kind}
+    lead = {"stack": (c.get("layers"), c["heads"]), "stack_prefill": (c.get("layers"), c["heads"]),
+            "grouped": (c.get("batch"), c["heads"])}.get(kind, (c["heads"],))
+    if kind in ("prefill", "stack_prefill"):
+        k, v = (_values((c["tokens"],) + lead + (dim,), dist, gen) for _ in range(2))
+    else:
+        scale = _fill(append, c["context"], lead, dim, dist, gen)
+        k, v = (_values(lead + (dim,), dist, gen, scale) for _ in range(2))
     if kind in ("engine", "window"):
-        kw = dict(v_mass=0.0, hybrid_thresh=0) if c.get("dense") else {}
-        cap = c["context"] if kind == "engine" else 4096
-        e = adaptq_b200.Engine(dim, c["heads"], c["k_bits"], c["v_bits"], cap, 42, **kw)
-        _fill(e.append_many, c["context"], (c["heads"],), dim, dist, gen)
-        s["engine"] = e
-        s["k"], s["v"], s["q"] = (_values((c["heads"], dim), dist, gen) for _ in range(3))
+        return k, v, _values(lead + (dim,), dist, gen)
+    q = torch.randn(lead[:-1] + (lead[-1] * c.get("q_per_kv", 1), dim), device="cuda", generator=gen)
+    if c.get("bf16"):
+        k, v, q = (t.to(torch.bfloat16) for t in (k, v, q))
+    return k, v, q
+
+
+def _batch_seeds(heads):
+    """Engines of many layers and sequences behind one handle: seed 42 ^ layer, 8 heads per layer."""
+    return [((42 ^ (i // 8 % 32)) ^ (i % 8 * 0xDEADBEEFCAFE)) & SEED_MASK for i in range(heads)]
+
+
+def _k_bits(case):
+    """Key bits per layer: a stack's layer 0 keeps FP32 keys."""
+    return [16] + [case["k_bits"]] * (case["layers"] - 1)
+
+
+def prepare(case, seed):
+    c, kind, dim = dict(case), case["kind"], case["dim"]
+    s = {"kind": kind}
+    if kind in ("engine", "window", "prefill"):
+        kw = dict(v_mass=0.0, hybrid_thresh=0) if c.get("dense", kind == "prefill") else {}
+        cap = {"engine": c.get("context"), "window": 4096, "prefill": c.get("tokens")}[kind]
+        s["engine"] = adaptq_b200.Engine(dim, c["heads"], c["k_bits"], c["v_bits"], cap, 42, **kw)
+        append = s["engine"].append_many
     elif kind in ("stack", "stack_prefill"):
-        lead = (c["layers"], c["heads"])
-        kb = [16] + [c["k_bits"]] * (c["layers"] - 1)  # layer 0 keeps FP32 keys
-        n = c["context"] if kind == "stack" else c["tokens"]
-        s["stack"] = adaptq_b200.LayerStack(c["layers"], c["heads"], dim, k_bits=kb, v_bits=c["v_bits"], capacity=n, seed=42,
-                                            v_mass=0.0, hybrid_thresh=0)
-        if kind == "stack":
-            scale = _fill(s["stack"].append, n, lead, dim, dist, gen)
-            s["k"], s["v"] = (_values(lead + (dim,), dist, gen, scale) for _ in range(2))
-        else:
-            s["k"], s["v"] = (_values((n,) + lead + (dim,), dist, gen) for _ in range(2))
-        s["q"] = torch.randn(lead + (dim,), device="cuda", generator=gen)
-        s["out"] = torch.empty_like(s["q"])
+        s["stack"] = adaptq_b200.LayerStack(c["layers"], c["heads"], dim, k_bits=_k_bits(c), v_bits=c["v_bits"],
+                                            capacity=c["context"] if kind == "stack" else c["tokens"], seed=42, v_mass=0.0,
+                                            hybrid_thresh=0)
+        append = s["stack"].append
     elif kind in ("batch", "long"):
-        heads, n = c["heads"], c["context"]
-        kw = {"seed": 42}
-        if kind == "batch":  # engines of many layers and sequences behind one handle: seed 42 ^ layer, 8 heads per layer
-            kw = {"seeds": [((42 ^ (i // 8 % 32)) ^ (i % 8 * 0xDEADBEEFCAFE)) & SEED_MASK for i in range(heads)]}
-        ctx = adaptq_b200.MHAContext(heads, dim, c["k_bits"], c["v_bits"], n, v_mass=0.0, hybrid_thresh=0, **kw)
-        _fill(ctx.append_all, n, (heads,), dim, dist, gen)
-        s["ctx"] = ctx
-        s["k"], s["v"] = (_values((heads, dim), dist, gen) for _ in range(2))
-        s["q"] = torch.randn((heads, dim), device="cuda", generator=gen)
-        s["out"] = torch.empty_like(s["q"])
-    elif kind == "grouped":
-        b, h, g = c["batch"], c["heads"], c["q_per_kv"]
+        kw = {"seeds": _batch_seeds(c["heads"])} if kind == "batch" else {"seed": 42}
+        s["ctx"] = adaptq_b200.MHAContext(c["heads"], dim, c["k_bits"], c["v_bits"], c["context"], v_mass=0.0, hybrid_thresh=0, **kw)
+        append = s["ctx"].append_all
+    else:  # grouped
         kw = dict(v_mass=0.0, hybrid_thresh=0) if c["dense"] else {}
-        m = adaptq_b200.BatchedAdaptQAttention(dim, h, b, c["k_bits"], c["v_bits"], c["context"], 42, q_per_kv=g, **kw)
-        step = max(1, 2**26 // (b * h * dim))
-        for t in range(0, c["context"], step):
-            shape = (b, min(step, c["context"] - t), h, dim)
-            m.prefill(_values(shape, dist, gen), _values(shape, dist, gen))
-        s["module"] = m
-        dt = torch.bfloat16 if c["bf16"] else torch.float32
-        s["k"], s["v"] = (_values((b, h, dim), dist, gen).to(dt) for _ in range(2))
-        s["q"] = torch.randn((b, h * g, dim), device="cuda", generator=gen).to(dt)
-    else:  # prefill
-        heads, n = c["heads"], c["tokens"]
-        s["engine"] = adaptq_b200.Engine(dim, heads, c["k_bits"], c["v_bits"], n, 42, v_mass=0.0, hybrid_thresh=0)
-        s["k"], s["v"] = (_values((n, heads, dim), dist, gen) for _ in range(2))
-        s["q"] = torch.randn((heads, dim), device="cuda", generator=gen)
+        m = s["module"] = adaptq_b200.BatchedAdaptQAttention(dim, c["heads"], c["batch"], c["k_bits"], c["v_bits"], c["context"], 42,
+                                                             q_per_kv=c["q_per_kv"], **kw)
+        append = lambda k, v: m.prefill(k.transpose(0, 1), v.transpose(0, 1))  # noqa: E731
+    s["k"], s["v"], s["q"] = _draw_inputs(c, seed, append)
+    s["out"] = torch.empty_like(s["q"])
     return s
 
 
@@ -263,3 +265,116 @@ def tolerance(case):
     if case["dist"] in ("student3", "student4", "outlier"):
         return {"rel": 4e-6, "max": 2e-4}  # 8.3e-7 and 3.7e-5 measured: some logits are in the hundreds
     return {"rel": 4e-6, "max": 4e-5}      # 8.5e-7 and 3.8e-6 measured
+
+
+# ---------------------------------------------------------------------------
+# the same in 64 bits
+# ---------------------------------------------------------------------------
+# Lloyd-Max centroids of N(0, 1) for 2, 3 and 4 bits (upper halves; the codebooks are odd)
+_CENTROIDS = {2: [0.4528, 1.5104], 3: [0.2451, 0.7560, 1.3439, 2.1529],
+              4: [0.1258, 0.3795, 0.6402, 0.9138, 1.2016, 1.5105, 1.8944, 2.4008]}
+
+
+def _signs(seeds, padded):
+    """Rademacher signs of each seed: one xorshift64 step per coordinate, +1 where the low bit is set."""
+    s = np.array([x if x else 0xDEADBEEFCAFE1234 for x in seeds], dtype=np.uint64)
+    out = np.empty((len(seeds), padded), dtype=np.float32)
+    for j in range(padded):
+        s ^= s << np.uint64(13)
+        s ^= s >> np.uint64(7)
+        s ^= s << np.uint64(17)
+        out[:, j] = np.where(s & np.uint64(1), 1.0, -1.0)
+    return torch.from_numpy(out).cuda()
+
+
+def _hadamard(x):
+    """Unnormalised Walsh-Hadamard butterflies over the last axis, stage by stage."""
+    shape, p, h = x.shape, x.shape[-1], 1
+    while h < p:
+        y = x.reshape(-1, p // (2 * h), 2, h)
+        x = torch.stack((y[:, :, 0] + y[:, :, 1], y[:, :, 0] - y[:, :, 1]), 2).reshape(shape)
+        h *= 2
+    return x
+
+
+def _pad(x, padded):
+    return torch.nn.functional.pad(x, (0, padded - x.shape[-1]))
+
+
+def _quantise(x, signs, bits):
+    """Rows as the cache holds them: levels and scale.  What is stored is defined in 32-bit steps
+    (norm summed in order, scale, signs, butterflies, two scalings, thresholds), so this part is 32 bits."""
+    total = torch.zeros_like(x[..., 0])
+    for j in range(x.shape[-1]):
+        total = total + x[..., j] * x[..., j]
+    norm = torch.sqrt(total + 1e-12)
+    padded = signs.shape[-1]
+    root = np.sqrt(np.float32(padded))
+    y = _hadamard(_pad(x * (torch.ones_like(norm) / norm)[..., None], padded) * signs)
+    y = (y * float(np.float32(1) / root)) * float(root)
+    half = np.array(_CENTROIDS[bits], dtype=np.float32)
+    cb = np.concatenate((-half[::-1], half))
+    thr = torch.from_numpy((cb[:-1] + cb[1:]) * np.float32(0.5)).cuda()
+    return torch.bucketize(y, thr, right=True).to(torch.uint8), norm, torch.from_numpy(cb.astype(np.float64)).cuda()
+
+
+def _attend(q, keys, v_levels, v_scale, v_cb, signs, dim):
+    """softmax(q . keys / sqrt(dim)) over (head, token) rows, values decoded; all in 64 bits.
+    q (heads, g, p); keys (heads, tokens, p)."""
+    p = signs.shape[-1]
+    w = torch.softmax(q @ keys.transpose(1, 2) / math.sqrt(dim), dim=-1)
+    acc = (w * v_scale.double()[:, None]) @ v_cb[v_levels.long()]
+    return (_hadamard(acc) / p * signs[:, None].double())[..., :dim]
+
+
+def exact(case, seed):
+    """Attention over the stored rows in 64 bits; the rows themselves are what 32-bit quantisation
+    defines.  None for sparse V (where its running 32-bit sum stops decides what is summed) and for the largest cache."""
+    c, kind, dim = case, case["kind"], case["dim"]
+    n = c.get("context", c.get("tokens"))
+    layers, g = c.get("layers", 1), c.get("q_per_kv", 1)
+    inst = c["heads"] * layers * c.get("batch", 1)
+    if not c.get("dense", True) or inst * n * dim > 2**31:
+        return None
+    parts = []
+    k, v, q = _draw_inputs(c, seed, lambda kk, vv: parts.append((kk.reshape(-1, inst, dim), vv.reshape(-1, inst, dim))))
+    if kind in ("prefill", "stack_prefill"):
+        parts = [(k.reshape(-1, inst, dim), v.reshape(-1, inst, dim))]
+    q = q.reshape(inst, g, dim).double()
+    if kind == "window":  # up to 512 tokens are attended to as they came
+        ks, vs = (torch.cat([x[i] for x in parts]).double().transpose(0, 1) for i in range(2))
+        w = torch.softmax(q @ ks.transpose(1, 2) / math.sqrt(dim), dim=-1)
+        return (w @ vs).reshape(c["heads"], dim)
+    if kind in ("engine", "stack", "batch", "grouped"):  # the ring is full: the new token takes the oldest one's place
+        parts[0] = tuple(x[1:] for x in parts[0])
+        parts.append((k.float().reshape(1, inst, dim), v.float().reshape(1, inst, dim)))
+    heads = c["heads"]
+    seeds = _batch_seeds(heads) if kind == "batch" else [
+        ((42 ^ l) ^ (i * 0xDEADBEEFCAFE)) & SEED_MASK for l in range(layers) for i in range(heads)] * c.get("batch", 1)
+    padded = _padded(dim)
+    signs = _signs(seeds, padded)
+    bits = [b for b in (_k_bits(c) if kind in ("stack", "stack_prefill") else [c["k_bits"]]) for _ in range(heads)]
+    out = torch.empty((inst, g, dim), dtype=torch.float64, device="cuda")
+    step = max(1, 2**24 // (n * padded))
+    for a in range(0, inst, step):
+        b = min(inst, a + step)
+        ks, vs = (torch.cat([x[i][:, a:b] for x in parts]).transpose(0, 1) for i in range(2))
+        sg = signs[a:b]
+        vl, vsc, vcb = _quantise(vs, sg[:, None], c["v_bits"])
+        kb = [bits[i] if len(bits) > heads else bits[0] for i in range(a, b)]
+        for fp32 in (True, False):
+            rows = [i for i, x in enumerate(kb) if (x == 16) == fp32]
+            if not rows:
+                continue
+            r = torch.tensor(rows, device="cuda")
+            qq = q[a:b][r]
+            if fp32:
+                keys = ks[r].double()
+            else:
+                kl, ksc, kcb = _quantise(ks[r], sg[r][:, None], c["k_bits"])
+                keys = kcb[kl.long()] * (ksc.double() / padded)[..., None]
+                qq = _hadamard(_pad(qq, padded) * sg[r][:, None].double())
+            out[a:b][r] = _attend(qq, keys, vl[r], vsc[r], vcb, sg[r], dim)
+    shape = {"stack": (layers, heads, dim), "stack_prefill": (layers, heads, dim),
+             "grouped": (c.get("batch"), heads * g, dim)}.get(kind, (heads, dim))
+    return out.reshape(shape)
