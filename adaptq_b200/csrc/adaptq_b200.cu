@@ -10,6 +10,7 @@
 #include "compute_general.cuh"
 #include "compute_sparse.cuh"
 #include "compute_stream.cuh"
+#include "compute_group.cuh"
 #include "runtime_v2.cuh"
 
 #include <algorithm>
@@ -121,7 +122,7 @@ struct Group {
   // device staging for host-pointer calls, and scratch for partials / sparse V
   void *d_stage = nullptr; size_t stage_bytes = 0;
   void *h_stage = nullptr; size_t h_stage_bytes = 0;
-  void *d_scratch_base = nullptr; // header + scratch, one allocation
+  void *d_scratch_base = nullptr; // header + scratch, one allocation (nullptr while they lie behind the key scales)
   void *d_scratch = nullptr; size_t scratch_bytes = 0;
   int *d_counters = nullptr;
   int *d_status = nullptr;
@@ -245,6 +246,19 @@ void sign_words_for(uint64_t seed, int padded, uint32_t *words, int n_words) {
   }
 }
 
+// Scratch = a zeroed header of arrival counters (kernels that use them leave them at
+// zero) followed by the space for partials / sparse-V work arrays.
+constexpr size_t SCRATCH_HEADER = 65536;
+constexpr int MAX_COUNTED_ITEMS = (int)(SCRATCH_HEADER / sizeof(int));
+
+// Caches whose grouped queries may go to compute_group_kernel (dense V, 2- to 4-bit rows of padded
+// dimension 64 or 128) get room for its pieces' partials with the handle, behind the key scales,
+// where that is below a tenth of the cache: a later cudaMalloc costs the first call half a millisecond.
+bool group_rows(const CacheView &c) { return (c.padded == 64 || c.padded == 128) && c.k_bits <= 4 && c.v_bits <= 4; }
+size_t group_scratch_bytes(const CacheView &c, int runs, int per_group) {
+  return (size_t)runs * 2 * per_group * (2 + c.padded) * sizeof(float);
+}
+
 Group *create_group(const char *fn, const char *bad_args_msg, int n_heads, const uint64_t *seeds, int dim,
                     int k_bits, int v_bits, int capacity, float v_mass, int hyb, bool single) {
   if (n_heads <= 0 || dim <= 0 || !valid_bits(k_bits) || !valid_bits(v_bits) || capacity < 0 || hyb < 0) {
@@ -281,10 +295,13 @@ Group *create_group(const char *fn, const char *bad_args_msg, int n_heads, const
   c.sign_words = (P + 31) / 32;
   c.mirror_stride = (size_t)hyb * 2 * dim;
   const char *what = fn;
+  const size_t scale_bytes = (size_t)c.s_stride * n_heads * 4;
+  size_t room = group_scratch_bytes(c, GQ_GROUPS * g->sm_count, 4);
+  if (!group_rows(c) || v_mass > 0.f || (double)n_heads * capacity * (c.k_row + c.v_row + 8) < 10. * (room + SCRATCH_HEADER)) room = 0;
   bool ok = alloc((void **)&c.k_slab, c.k_stride * n_heads, g, what) &&
             alloc((void **)&c.v_slab, c.v_stride * n_heads, g, what) &&
-            alloc((void **)&c.k_scale, (size_t)c.s_stride * n_heads * 4, g, what) &&
-            alloc((void **)&c.v_scale, (size_t)c.s_stride * n_heads * 4, g, what) &&
+            alloc((void **)&c.k_scale, scale_bytes + (room ? SCRATCH_HEADER + room : 0), g, what) &&
+            alloc((void **)&c.v_scale, scale_bytes, g, what) &&
             alloc((void **)&c.signs, (size_t)c.sign_words * n_heads * 4, g, what) &&
             alloc((void **)&g->d_status, 16, g, what);
   if (ok && hyb > 0) ok = alloc((void **)&c.mirror, c.mirror_stride * n_heads * 4, g, what);
@@ -300,7 +317,14 @@ Group *create_group(const char *fn, const char *bad_args_msg, int n_heads, const
     fill_f32_kernel<<<(int)std::min<size_t>((ns + 255) / 256, 4096), 256>>>(c.k_scale, ns, 1.0f);
     fill_f32_kernel<<<(int)std::min<size_t>((ns + 255) / 256, 4096), 256>>>(c.v_scale, ns, 1.0f);
     g_launches += 2;
-    e = cudaDeviceSynchronize();
+    if (room) { // scale_bytes is a multiple of 128
+      char *base = reinterpret_cast<char *>(c.k_scale) + scale_bytes;
+      e = cudaMemsetAsync(base, 0, SCRATCH_HEADER);
+      g->d_counters = reinterpret_cast<int *>(base);
+      g->d_scratch = base + SCRATCH_HEADER;
+      g->scratch_bytes = room;
+    }
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
   }
   if (e != cudaSuccess) {
     set_error("%s: CUDA error during set-up: %s", fn, cudaGetErrorString(e));
@@ -345,10 +369,6 @@ bool ensure_stage(Group *g, size_t dev_bytes, size_t host_bytes) {
   return true;
 }
 
-// Scratch = a zeroed header of arrival counters (kernels that use them leave them at
-// zero) followed by the space for partials / sparse-V work arrays.
-constexpr size_t SCRATCH_HEADER = 65536;
-constexpr int MAX_COUNTED_ITEMS = (int)(SCRATCH_HEADER / sizeof(int));
 bool ensure_scratch(Group *g, size_t bytes) {
   if (bytes <= g->scratch_bytes) return true;
   CUDA_TRY(cudaStreamSynchronize(g->stream), "scratch");
@@ -860,10 +880,91 @@ bool launch_stream(Group *g, const ComputeLaunch &ca, bool want_partial_out, flo
   return true;
 }
 
+// ---- grouped queries --------------------------------------------------------
+template <int KB, int VB, int P, int NT>
+bool launch_group_t(Group *g, const GroupLaunch &a, int grid) {
+  static int configured[MAX_DEVICES] = {};
+  auto kern = compute_group_kernel<KB, VB, P, NT>;
+  constexpr size_t SMEM = GroupPlan<KB, VB, P, NT>::SMEM;
+  if (!ensure_smem_limit(kern, configured, g->device, SMEM, "compute")) return false;
+  launch_attention(g, kern, dim3((unsigned)grid), GQ_THREADS, SMEM, a);
+  ++g_launches;
+  CUDA_TRY(launch_status(), "compute");
+  return true;
+}
+template <int KB, int P, int NT>
+bool launch_group_v(Group *g, const GroupLaunch &a, int grid) {
+  switch (a.c.v_bits) {
+  case 2: return launch_group_t<KB, 2, P, NT>(g, a, grid);
+  case 3: return launch_group_t<KB, 3, P, NT>(g, a, grid);
+  default: return launch_group_t<KB, 4, P, NT>(g, a, grid);
+  }
+}
+template <int P, int NT>
+bool launch_group_kv(Group *g, const GroupLaunch &a, int grid) {
+  switch (a.c.k_bits) {
+  case 2: return launch_group_v<2, P, NT>(g, a, grid);
+  case 3: return launch_group_v<3, P, NT>(g, a, grid);
+  default: return launch_group_v<4, P, NT>(g, a, grid);
+  }
+}
+
+// Calls with several queries per head that compute_group_kernel takes.  Its time grows little with
+// the queries (512 heads x 4096 tokens, K4/V2, dim 128: 84 / 113 / 197 us at 2 / 4 / 8 queries, where
+// the streaming kernel, which walks the cache once per query, takes 113 / 213 / 414), but a launch
+// costs about 8 us more.  Measured crossings, in packed bytes times queries: 128 heads x 2048 x 2
+// queries (55 MB) 29 us against 27, 334 x 3001 x 2 (206 MB) 64 against 93; 64 heads x 1500 tokens of
+// dim 64 x 4 queries (25 MB) 25 against 21, x 7 (43 MB) 27 against 33.
+bool group_applies(const CacheView &c, long long heads, int nq, int n) {
+  if (nq < 2 || !group_rows(c)) return false;
+  const double work = (double)heads * nq * n * (c.k_row + c.v_row + 8);
+  return work >= (nq == 2 ? 80e6 : 40e6);
+}
+
+bool launch_group(Group *g, const ComputeLaunch &ca) {
+  const CacheView &c = g->c;
+  GroupLaunch a{};
+  a.c = c; a.q = ca.q; a.out = ca.out; a.head0 = ca.head0; a.heads_in_call = ca.heads_in_call; a.nq = ca.nq;
+  a.n = ca.n; a.status = g->d_status;
+  const int nt = a.nq <= 2 ? 1 : 2; // tensor-core column tiles, two queries each
+  a.groups_per_head = (a.nq + 2 * nt - 1) / (2 * nt);
+  a.per_group = (a.nq + a.groups_per_head - 1) / a.groups_per_head;
+  const long long items = (long long)a.heads_in_call * a.groups_per_head;
+  const long long items_base = (long long)a.heads_in_call * a.nq;
+  // Heads are cut anywhere on 64-token boundaries, so that all groups get equal shares.  They stay
+  // whole where there are more queries than arrival counters (then there are many heads), and where
+  // room for the pieces' partials cannot be had: no memory, or a stream capture under way.
+  bool cut = items_base <= MAX_COUNTED_ITEMS;
+  int grid = g->sm_count;
+  if (cut) {
+    a.unit_tokens = GQ_UNIT;
+    a.units = (a.n + GQ_UNIT - 1) / GQ_UNIT;
+    const long long total = items * a.units;
+    // a run of at least 256 tokens, and of a 16th of a head: one warp merges a head's pieces
+    const long long shortest = std::max<long long>(4, a.units / 16);
+    grid = (int)std::max<long long>(1, std::min<long long>(grid, total / (GQ_GROUPS * shortest)));
+    const size_t bytes = group_scratch_bytes(c, grid * GQ_GROUPS, a.per_group); // at most 1.2 MB
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (bytes > g->scratch_bytes && (cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)) cut = false;
+    else if (!ensure_scratch(g, bytes)) { clear_error(); cut = false; }
+    a.partial = static_cast<float *>(g->d_scratch);
+    a.counters = g->d_counters;
+  }
+  if (!cut) {
+    a.unit_tokens = a.n;
+    a.units = 1;
+    grid = (int)std::max<long long>(1, std::min<long long>(g->sm_count, items / GQ_GROUPS));
+  }
+  if (c.padded == 128) return nt == 1 ? launch_group_kv<128, 1>(g, a, grid) : launch_group_kv<128, 2>(g, a, grid);
+  return nt == 1 ? launch_group_kv<64, 1>(g, a, grid) : launch_group_kv<64, 2>(g, a, grid);
+}
+
 bool launch_general_or_stream(Group *g, ComputeLaunch &a, bool want_partial_out, float *partial_out) {
   const CacheView &c = g->c;
   const int policy = g_policy.load();
   const bool can_stream = !a.use_mirror && stream_supported(c);
+  if (!a.use_mirror && !want_partial_out && policy != 1 && (can_stream || policy == 0) && group_applies(c, a.heads_in_call, a.nq, a.n))
+    return launch_group(g, a);
   if (can_stream && policy != 1) return launch_stream(g, a, want_partial_out, partial_out);
   if (policy == 2) { set_error("compute: shape not covered by the streaming kernel"); return false; }
   return launch_general(g, a, want_partial_out, partial_out);

@@ -1,0 +1,88 @@
+"""Grouped queries on the tensor-core kernel (compute_group.cuh) against the CPU oracle (a few
+heads) and the general kernel (all heads), at the edges of its tiles, chunks and work split.
+Tolerances: helpers.RTOL / helpers.ATOL for both, as for every other attention kernel."""
+import numpy as np
+import pytest
+
+from helpers import CpuHeads, assert_close
+
+pytestmark = pytest.mark.gpu
+
+# dim, k_bits, v_bits, tokens, queries per head, capacity (0: tokens)
+CASES = [
+    (128, 4, 2, 2, 4, 0),        # two tokens; more queries than arrival counters, so heads stay whole
+    (128, 4, 4, 17, 3, 0),       # one row past a tile of 16
+    (64, 2, 3, 33, 5, 0),        # one past the V stream's 32; two query groups, 3 + 2
+    (128, 3, 3, 64, 2, 0),       # exactly one unit of the split
+    (64, 4, 4, 65, 8, 0),
+    (128, 2, 4, 127, 7, 0),
+    (64, 3, 2, 129, 4, 0),       # one past a stage
+    (128, 4, 3, 1535, 4, 0),     # around the chunk of three and four queries
+    (64, 4, 2, 1537, 6, 0),
+    (128, 2, 2, 2049, 2, 0),     # one past the chunk of two
+    (64, 2, 2, 3001, 4, 0),      # 2-bit keys at 64: not a shape of the streaming kernel
+    (128, 3, 2, 40000, 3, 0),    # few heads, many pieces each
+    (64, 3, 4, 1100, 2, 1024),   # wrapped ring
+    (96, 4, 2, 700, 4, 0),       # padded dimension
+]
+
+
+@pytest.mark.parametrize("dim,kb,vb,n,nq,cap", CASES)
+def test_grouped_queries(gpu_lib, orc, dim, kb, vb, n, nq, cap):
+    import torch
+    from adaptq_b200 import MHAContext
+    padded = 64 if dim == 64 else 128
+    live = min(n, cap or n)
+    row = padded * (kb + vb) // 8 + 8
+    heads = max(3, int((80e6 if nq == 2 else 40e6) / (nq * live * row)) + 1)  # just above the size where the kernel is chosen
+    gen = torch.Generator(device="cuda").manual_seed(dim + 7 * kb + 11 * vb + n)
+    rnd = lambda *s: torch.randn(s, device="cuda", generator=gen)  # noqa: E731
+    k, v, q = rnd(n, heads, dim), rnd(n, heads, dim), rnd(heads, nq, dim)
+    k[torch.rand(k.shape, device="cuda", generator=gen) < 0.002] *= 10
+    seeds = [(42 ^ (i % 5)) for i in range(heads)]
+    ctx = MHAContext(heads, dim, kb, vb, cap or n, v_mass=0.0, hybrid_thresh=0, seeds=seeds)
+    ctx.append_all(k, v)
+    before = gpu_lib.adaptq_kernel_launches()
+    out = ctx.compute_all(q)
+    assert gpu_lib.adaptq_kernel_launches() - before == 1, "one launch for all queries"
+    assert torch.equal(out, ctx.compute_all(q)), "integer sums: the same bits every time"
+    ctx.synchronize()
+    pick = [0, heads // 2, heads - 1]
+    cpu = CpuHeads(orc, 3, dim, kb, vb, cap or n, 0, seeds=[seeds[i] for i in pick])
+    cpu.append_many(k[:, pick].cpu().numpy(), v[:, pick].cpu().numpy())
+    assert_close(out[pick].cpu().numpy(), cpu.compute_batch(q[pick].cpu().numpy()), "against the oracle")
+    try:
+        gpu_lib.adaptq_set_kernel_policy(1)
+        ref = ctx.compute_all(q)
+    finally:
+        gpu_lib.adaptq_set_kernel_policy(0)
+    assert_close(out.cpu().numpy(), ref.cpu().numpy(), "against the general kernel")
+
+
+def test_grouped_queries_non_finite(gpu_lib):
+    """A NaN query gives NaN outputs for itself alone; an infinite value row for its head alone; a
+    zero query averages."""
+    import torch
+    from adaptq_b200 import MHAContext
+    heads, dim, n, nq = 300, 128, 400, 4
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    k, v, q = (torch.randn(s, device="cuda", generator=gen) for s in ((n, heads, dim), (n, heads, dim), (heads, nq, dim)))
+    v[7, 1] = float("inf")
+    q[0, 2] = 0.0
+    ctx = MHAContext(heads, dim, 4, 2, n, seed=1, v_mass=0.0, hybrid_thresh=0)
+    ctx.append_all(k, v)
+    want = ctx.compute_all(q)
+    q[0, 1, 5] = float("nan")
+    got = ctx.compute_all(q)
+    try:
+        gpu_lib.adaptq_set_kernel_policy(1)
+        ref = ctx.compute_all(q)
+    finally:
+        gpu_lib.adaptq_set_kernel_policy(0)
+    assert torch.isnan(got[0, 1]).all() and torch.isnan(got[1]).all()
+    rest = torch.isfinite(ref)
+    assert torch.equal(torch.isfinite(got), rest)
+    assert_close(got[rest].cpu().numpy(), ref[rest].cpu().numpy(), "against the general kernel")
+    same = torch.ones_like(rest)
+    same[0, 1] = same[1] = False
+    assert torch.equal(got[same], want[same])
