@@ -11,6 +11,7 @@
 #include "compute_sparse.cuh"
 #include "compute_stream.cuh"
 #include "compute_group.cuh"
+#include "compute_window.cuh"
 #include "runtime_v2.cuh"
 
 #include <algorithm>
@@ -447,9 +448,9 @@ bool ensure_smem_limit(K kern, int (&slot)[MAX_DEVICES], int device, size_t byte
 // the launch carries the programmatic-stream-serialisation attribute: the kernel may start
 // while the append still runs and waits inside (griddep_wait) before it reads the cache.
 template <typename Kern, typename... Args>
-void launch_attention(Group *g, Kern kern, dim3 grid, int threads, size_t smem, Args... args) {
+void launch_attention_clusters(Group *g, Kern kern, dim3 grid, int cluster, int threads, size_t smem, Args... args) {
   const bool pdl = g->append_ticket.exchange(~0ull) == g_launches.load();
-  if (!pdl) {
+  if (!pdl && cluster == 1) {
     kern<<<grid, threads, smem, g->stream>>>(args...);
     return;
   }
@@ -458,12 +459,25 @@ void launch_attention(Group *g, Kern kern, dim3 grid, int threads, size_t smem, 
   cfg.blockDim = dim3((unsigned)threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = g->stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
+  int n_attr = 0;
+  if (pdl) {
+    attr[n_attr].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n_attr++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[n_attr].id = cudaLaunchAttributeClusterDimension;
+    attr[n_attr].val.clusterDim.x = (unsigned)cluster;
+    attr[n_attr].val.clusterDim.y = 1;
+    attr[n_attr++].val.clusterDim.z = 1;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = (unsigned)n_attr;
   cudaLaunchKernelEx(&cfg, kern, args...); // the caller reads the launch status
+}
+template <typename Kern, typename... Args>
+void launch_attention(Group *g, Kern kern, dim3 grid, int threads, size_t smem, Args... args) {
+  launch_attention_clusters(g, kern, grid, 1, threads, smem, args...);
 }
 
 // ---------------------------------------------------------------------------
@@ -970,6 +984,18 @@ bool launch_general_or_stream(Group *g, ComputeLaunch &a, bool want_partial_out,
   return launch_general(g, a, want_partial_out, partial_out);
 }
 
+// The FP32 window on its own kernel (whole float4 rows up to 128 columns).
+bool window_applies(const CacheView &c) { return c.dim % 4 == 0 && c.dim <= WK_MAX_DIM; }
+bool launch_window(Group *g, const ComputeLaunch &a) {
+  int cluster = 1; // 64 tokens a block while the cluster lasts
+  while (cluster < WK_MAX_CLUSTER && cluster * WK_TOKENS < a.n) cluster *= 2;
+  const dim3 grid((unsigned)((long long)a.heads_in_call * a.nq * cluster));
+  launch_attention_clusters(g, window_kernel, grid, cluster, WK_THREADS, 0, a.c, a.q, a.out, a.head0, a.nq, a.n, a.status);
+  ++g_launches;
+  CUDA_TRY(launch_status(), "compute (window)");
+  return true;
+}
+
 // dq, dout on the device.  All heads of the call share `st`.
 bool compute_device(Group *g, const float *dq, float *dout, int head0, int heads_in_call, int nq, RingState st,
                     bool partial_out) {
@@ -988,6 +1014,7 @@ bool compute_device(Group *g, const float *dq, float *dout, int head0, int heads
   a.use_mirror = (c.hyb > 0 && st.size <= c.hyb && st.mirror == st.size) ? 1 : 0;
   const bool quant = c.k_bits != 16 && c.v_bits != 16;
   if (partial_out) return launch_general_or_stream(g, a, true, dout);
+  if (a.use_mirror && g_policy.load() == 0 && window_applies(c)) return launch_window(g, a);
   if (!a.use_mirror && c.v_mass > 0.f && quant) return launch_sparse(g, a);
   return launch_general_or_stream(g, a, false, nullptr);
 }

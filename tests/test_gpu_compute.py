@@ -365,3 +365,21 @@ def test_peer_merge_gives_up_when_a_rank_never_delivers(gpu_lib, orc):
     cpu.append_many(k, v)
     assert_close(ctx.compute_all(q).cpu().numpy(), cpu.compute(q.cpu().numpy()), "after the timed-out merge")
     ctx.synchronize()
+
+
+@pytest.mark.parametrize("dim,n,hyb,nq", [(64, 1, 512, 1), (128, 9, 512, 3), (128, 64, 512, 1), (80, 65, 512, 2), (4, 129, 512, 1), (96, 257, 512, 1),
+                                          (128, 512, 512, 4), (64, 1100, 1300, 1), (30, 70, 512, 1), (256, 70, 512, 1)])
+def test_window_matches_oracle(gpu_lib, orc, dim, n, hyb, nq):
+    """The FP32 window at the edges of its kernel's split (64 tokens a block, 8 a warp, clusters of 1 to 8),
+    and at dimensions that stay on the general kernel (30: no whole float4, 256: more than a warp's columns)."""
+    from adaptq_b200 import MHAContext
+    heads = 3
+    rng = np.random.default_rng(dim + n)
+    k, v = make_kv(rng, n, heads, dim, "normal_outlier")
+    q = rng.standard_normal((heads, nq, dim)).astype(np.float32)
+    ctx = MHAContext(heads, dim, 4, 4, 2048, seed=42, v_mass=0.95, hybrid_thresh=hyb)
+    cpu = CpuHeads(orc, heads, dim, 4, 4, 2048, 42, 0.95, hyb)
+    ctx.append_all(k, v)
+    cpu.append_many(k, v)
+    assert_close(ctx.compute_all(q), cpu.compute_batch(q), "window")
+    ctx.synchronize()
