@@ -47,7 +47,7 @@ template <int ITEMS> __device__ __forceinline__ int sp_pos(int tid, int k) { ret
 // Weights lie in [0, 1], so their IEEE bit patterns occupy 30 bits and order like integers; the
 // sort runs on the complemented pattern (ascending) with four least-significant-digit passes of
 // 8 bits.  A pass: every warp counts its digits (lanes with equal digits find each other with
-// votes on the digit's bits; the items of a warp are ranked k = 0, 1, ... in turn so that a running per-warp
+// match.any; the items of a warp are ranked k = 0, 1, ... in turn so that a running per-warp
 // count gives the rank among the warp's earlier items), the counts [digit][warp] are scanned in
 // that order over the block, and the pairs move to their ranks through s_w / s_tok.
 // Padding (weight 0 at positions >= n) ties with real zero weights and stays behind them.
@@ -69,15 +69,7 @@ __device__ __forceinline__ void block_sort_pairs(float (&key)[ITEMS], int (&val)
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
       const uint32_t d = (u[k] >> shift) & 255u;
-      // lanes with the same digit, bit by bit: match.any gives this in one instruction, but a slow one
-      // (sorting 2048 pairs: 20.2 thousand clocks with it, 13.1 with eight votes; 4096: 33 and 23)
-      uint32_t same = 0xffffffffu;
-#pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        const bool one = (d >> b) & 1u;
-        const uint32_t ones = __ballot_sync(0xffffffffu, one);
-        same &= one ? ones : ~ones;
-      }
+      const uint32_t same = __match_any_sync(0xffffffffu, d);
       uint32_t *slot = cnt + d * SP_CNT_PITCH + warp;
       const uint32_t before = *slot;
       __syncwarp();
@@ -100,8 +92,8 @@ __device__ __forceinline__ void block_sort_pairs(float (&key)[ITEMS], int (&val)
       }
       if (lane == 31) warp_tot[warp] = inc;
       __syncthreads();
-      static_assert(SP_WARPS <= 32, "one lane per earlier warp");
-      uint32_t base = inc - tsum + __reduce_add_sync(0xffffffffu, lane < warp ? warp_tot[lane] : 0u);
+      uint32_t base = inc - tsum;
+      for (int w = 0; w < warp; ++w) base += warp_tot[w];
 #pragma unroll
       for (int j = 0; j < SP_CNT_PER_THREAD; ++j) { cnt[e0 + j] = base; base += loc[j]; }
     }
@@ -152,35 +144,27 @@ __device__ __forceinline__ float sp_block_reduce(float v, float *red, bool is_ma
 
 // Upstream's sequential walk (attention.cpp:455-473): add arr[0], arr[1], ... while the running
 // mass is below `limit`; returns how many were added.  The sums are strictly sequential (that
-// fixes the cut), but the weights are not negative, so the mass never falls and the test need not
-// sit between two additions: eight additions run on, and only where the limit was reached among
-// them are their sums looked at one by one (about 5 clocks an element instead of 24).
+// fixes the cut); the values are fetched eight at a time ahead of the sum so that the chain is
+// one addition and one comparison per element, not a shared-memory round trip.
 __device__ __forceinline__ int walk_mass(const float *arr, int len, float limit, float &mass) {
-  int i = 0;
-  float x[8], nx[8];
+  int i = 0, cnt = 0;
+  bool open = true;
+  while (open && i < len) {
+    float x[8];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) nx[k] = k < len ? arr[k] : 0.f;
-  while (i + 8 <= len) {
-    float m[8];
+    for (int k = 0; k < 8; ++k) x[k] = arr[min(i + k, len - 1)];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = nx[k];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) nx[k] = arr[min(i + 8 + k, len - 1)]; // the next eight come during this chain
-    m[0] = __fadd_rn(mass, x[0]);
-#pragma unroll
-    for (int k = 1; k < 8; ++k) m[k] = __fadd_rn(m[k - 1], x[k]);
-    if (!(m[6] < limit && mass < limit)) { // the limit, or a NaN, before the last of the eight
-      int cnt = 0;
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        if (cnt == k && mass < limit) { mass = m[k]; ++cnt; }
-      return i + cnt;
+    for (int k = 0; k < 8; ++k) {
+      if (open && i + k < len && mass < limit) {
+        mass = __fadd_rn(mass, x[k]);
+        ++cnt;
+      } else {
+        open = false;
+      }
     }
-    mass = m[7];
     i += 8;
   }
-  for (; i < len && mass < limit; ++i) mass = __fadd_rn(mass, arr[i]);
-  return i;
+  return cnt;
 }
 
 // V rows of the first `count` sorted tokens, by words (padded dimension a multiple of 32).
@@ -197,28 +181,15 @@ __device__ __forceinline__ void sparse_v_words(const float *s_w, const int *s_to
 #pragma unroll
   for (int k = 0; k < UU::NCO; ++k) acc[k] = 0.f;
   const uint8_t *vunit = vbase + (size_t)u * (UU::WORDS * 4);
-  // Rows in batches, all of a batch's loads in flight before the first is used: no branch around a
-  // load, places past the end read slot 0 and weigh nothing.
-  constexpr int BATCH = BITS == 3 ? 4 : 8;
-  for (int i0 = tg; i0 < count; i0 += BATCH * TG) {
-    uint32_t w[BATCH][UU::WORDS];
-    float wt[BATCH], vs[BATCH];
+#pragma unroll 2
+  for (int i = tg; i < count; i += TG) {
+    const int tok = s_tok[i];
+    if (!AQ_CHECK(status, tok >= 0 && tok < c.cap, 15)) continue;
+    uint32_t w[UU::WORDS];
+    load_words_be<UU::WORDS>(vunit + (size_t)tok * c.v_row, w);
+    const float wt = s_w[i] * __ldg(vsc + tok) * isp;
 #pragma unroll
-    for (int b = 0; b < BATCH; ++b) {
-      const int i = i0 + b * TG;
-      const int tok = i < count ? s_tok[i] : 0;
-      const bool live = i < count && AQ_CHECK(status, tok >= 0 && tok < c.cap, 15);
-      const int slot = live ? tok : 0;
-      wt[b] = live ? s_w[i] : -1.f;
-      vs[b] = __ldg(vsc + slot);
-      load_words_be<UU::WORDS>(vunit + (size_t)slot * c.v_row, w[b]);
-    }
-#pragma unroll
-    for (int b = 0; b < BATCH; ++b) wt[b] = wt[b] != -1.f ? wt[b] * vs[b] * isp : 0.f; // weights are not negative
-#pragma unroll
-    for (int b = 0; b < BATCH; ++b)
-#pragma unroll
-      for (int k = 0; k < UU::NCO; ++k) acc[k] += wt[b] * s_cb[level_of<BITS, UU::WORDS>(w[b], k)];
+    for (int k = 0; k < UU::NCO; ++k) acc[k] += wt * s_cb[level_of<BITS, UU::WORDS>(w, k)];
   }
   v_fold_words<BITS, SP_THREADS>(acc, P, buf, vec);
 }
@@ -258,46 +229,6 @@ __device__ __forceinline__ void sparse_rotate_warp(const float *qp, const uint32
   const float back = sqrtf((float)P) * qn, isq = 1.f / sqrtf((float)P);
 #pragma unroll
   for (int e = 0; e < EPL; ++e) qr[EPL * lane + e] = v[e] * isq * back;
-}
-
-// Logits of this thread's rows (slots val[], positions below n) against the [coordinate][level]
-// table: 32 coordinates at a time, the words of up to eight rows fetched together, so that the
-// thread waits for memory once per 32 coordinates and not once per row.
-template <int BITS, int ITEMS>
-__device__ __forceinline__ void sparse_score_rows(float (&key)[ITEMS], const int (&val)[ITEMS], const uint8_t *kbase, const float *ksc,
-                                                  const float *lut, const CacheView &c, int n, float attn_s, int *status) {
-  constexpr int BATCH = ITEMS < 8 ? ITEMS : 8, L = 1 << BITS;
-  const int tid = threadIdx.x, P = c.padded;
-#pragma unroll
-  for (int k0 = 0; k0 < ITEMS; k0 += BATCH) {
-    bool live[BATCH];
-    int row[BATCH];
-    float s0[BATCH], s1[BATCH], ks[BATCH];
-#pragma unroll
-    for (int b = 0; b < BATCH; ++b) {
-      const int slot = val[k0 + b];
-      live[b] = sp_pos<ITEMS>(tid, k0 + b) < n && AQ_CHECK(status, slot >= 0 && slot < c.cap, 15);
-      row[b] = live[b] ? slot : 0; // places past the end score slot 0 and drop the result
-      s0[b] = s1[b] = 0.f;
-      ks[b] = ksc[row[b]];
-    }
-#pragma unroll 1
-    for (int g = 0; g < P / 32; ++g) {
-      uint32_t w[BATCH][BITS];
-#pragma unroll
-      for (int b = 0; b < BATCH; ++b) load_words_be<BITS>(kbase + (size_t)row[b] * c.k_row + g * 4 * BITS, w[b]);
-      const float *lt = lut + (size_t)g * 32 * L;
-#pragma unroll
-      for (int b = 0; b < BATCH; ++b)
-#pragma unroll
-        for (int k = 0; k < 32; k += 2) {
-          s0[b] += lt[k * L + level_of<BITS, BITS>(w[b], k)];
-          s1[b] += lt[(k + 1) * L + level_of<BITS, BITS>(w[b], k + 1)];
-        }
-    }
-#pragma unroll
-    for (int b = 0; b < BATCH; ++b) key[k0 + b] = live[b] ? (s0[b] + s1[b]) * attn_s * ks[b] : -INFINITY;
-  }
 }
 
 template <int ITEMS>
@@ -344,9 +275,17 @@ __global__ void __launch_bounds__(SP_THREADS) sparse_fused_kernel(const float *l
     const uint8_t *kbase = c.k_slab + (size_t)h * c.k_stride;
     const float *ksc = c.k_scale + (size_t)h * c.s_stride;
     griddep_wait(); // the cache is read from here on
-    if (c.k_bits == 4) sparse_score_rows<4, ITEMS>(key, val, kbase, ksc, lut, c, n, attn_s, status);
-    else if (c.k_bits == 3) sparse_score_rows<3, ITEMS>(key, val, kbase, ksc, lut, c, n, attn_s, status);
-    else sparse_score_rows<2, ITEMS>(key, val, kbase, ksc, lut, c, n, attn_s, status);
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+      const int i = sp_pos<ITEMS>(tid, k);
+      key[k] = -INFINITY;
+      if (i < n && AQ_CHECK(status, val[k] >= 0 && val[k] < c.cap, 15)) {
+        const uint8_t *kr = kbase + (size_t)val[k] * c.k_row;
+        const float sum = c.k_bits == 4 ? score_row_words<4>(kr, lut, P)
+                          : c.k_bits == 3 ? score_row_words<3>(kr, lut, P) : score_row_words<2>(kr, lut, P);
+        key[k] = sum * attn_s * ksc[val[k]];
+      }
+    }
     __syncthreads(); // vec and the table are free again
   } else {
     const float *lg = logits + (size_t)item * w_stride;
