@@ -923,16 +923,66 @@ bool launch_group_kv(Group *g, const GroupLaunch &a, int grid) {
   }
 }
 
-// Calls with several queries per head that compute_group_kernel takes.  Its time grows little with
-// the queries (512 heads x 4096 tokens, K4/V2, dim 128: 84 / 113 / 197 us at 2 / 4 / 8 queries, where
-// the streaming kernel, which walks the cache once per query, takes 113 / 213 / 414), but a launch
-// costs about 8 us more.  Measured crossings, in packed bytes times queries: 128 heads x 2048 x 2
-// queries (55 MB) 29 us against 27, 334 x 3001 x 2 (206 MB) 64 against 93; 64 heads x 1500 tokens of
-// dim 64 x 4 queries (25 MB) 25 against 21, x 7 (43 MB) 27 against 33.
-bool group_applies(const CacheView &c, long long heads, int nq, int n) {
+// How a call is cut for compute_group_kernel.  Heads are cut anywhere on 64-token boundaries, so
+// that all groups get equal shares; they stay whole where there are more queries than arrival
+// counters (then there are many heads).
+struct GroupCut {
+  int nt, groups_per_head, per_group; // tensor-core column tiles (two queries each), query groups of a head, queries of a group
+  long long items;                    // (head, query group) pairs
+  int units, grid;                    // units per item, blocks
+  bool cut;
+};
+GroupCut group_cut(int sm_count, long long heads, int nq, int n) {
+  GroupCut p;
+  p.nt = nq <= 2 ? 1 : 2;
+  p.groups_per_head = (nq + 2 * p.nt - 1) / (2 * p.nt);
+  p.per_group = (nq + p.groups_per_head - 1) / p.groups_per_head;
+  p.items = heads * p.groups_per_head;
+  p.cut = heads * nq <= MAX_COUNTED_ITEMS;
+  p.units = p.cut ? (n + GQ_UNIT - 1) / GQ_UNIT : 1;
+  // a run of at least 256 tokens, and of a 16th of a head: one warp merges a head's pieces
+  const long long shortest = p.cut ? std::max(4, p.units / 16) : 1;
+  p.grid = (int)std::max<long long>(1, std::min<long long>(sm_count, p.items * p.units / (GQ_GROUPS * shortest)));
+  return p;
+}
+
+// Calls with several queries per head that compute_group_kernel takes: where it is expected to be
+// the faster one.  Its time is that of its longest run plus the ends of the segments in it; the
+// streaming kernel's is that of its waves of spans, each walked once per query.  The constants (us)
+// are fitted to 1500 pairs of measurements (1 to 16384 heads, 20 to 524288 tokens, 2 to 8 queries, all
+// widths, both dimensions); of those above the sizes below, the choice is within 6 % of the better
+// kernel but for 8 heads (24.6 us against 20.6 at worst), and within 5 % for 398 calls of other sizes.
+// Examples, streaming / this kernel, K4/V2,
+// dim 128, four queries: 512 heads x 4096 tokens 213 / 113, 32 x 16384 60 / 39, 32 x 4096 20 / 27,
+// 4 x 131072 58 / 107, 1 x 131072 26 / 107 (16 runs a head, so a few long heads leave most SMs idle).
+// Shapes that the streaming kernel does not have (2-bit keys at 64) come from the general kernel,
+// which loses by 1.4 to 3 times as soon as a fifth of the blocks have work (2 heads x 131072 x 8: 98
+// against 70, 1 x 524288 x 8: 143 against 243).
+bool group_applies(const CacheView &c, int sm_count, bool can_stream, long long heads, int nq, int n) {
   if (nq < 2 || !group_rows(c)) return false;
   const double work = (double)heads * nq * n * (c.k_row + c.v_row + 8);
-  return work >= (nq == 2 ? 80e6 : 40e6);
+  if (work < (nq == 2 ? 80e6 : 40e6)) return false; // packed bytes times queries; below, a launch costs more than it saves
+  const GroupCut p = group_cut(sm_count, heads, nq, n);
+  if (!can_stream) return 5 * p.grid >= sm_count;
+  const int runs = GQ_GROUPS * p.grid;
+  double run, segments; // of the longest run: units, and pieces of heads
+  if (p.cut) {
+    const long long total = p.items * p.units;
+    run = (double)total / runs;
+    const bool aligned = total % runs == 0 && ((total / runs) % p.units == 0 || p.units % (total / runs) == 0);
+    segments = aligned ? std::max(1., run / p.units) : std::min(std::max(1., run), run / p.units + 1.);
+  } else {
+    segments = (double)((p.items + runs - 1) / runs);
+    run = segments * ((n + GQ_UNIT - 1) / GQ_UNIT);
+  }
+  const bool two = p.nt == 1, narrow = c.padded == 64;
+  const double here = 9.7 + (two ? 4.5 : 8.7) * segments + (narrow ? (two ? 3.8 : 4.6) : (two ? 7.3 : 10.9)) * run * GQ_UNIT * 1e-3;
+  int n_splits, span;
+  plan_spans(n, (int)(heads * nq), sm_count, n_splits, span);
+  const long long waves = (heads * nq * n_splits + sm_count - 1) / sm_count;
+  const int lookups = c.padded / 4 * ((c.k_bits == 2 ? 1 : 2) + (c.v_bits == 2 ? 1 : 2)); // table reads and bucket adds per token
+  const double stream = 6.8 + (double)waves * (3.6 + 0.026 * lookups * std::min(span, n) * 1e-3);
+  return here < stream;
 }
 
 bool launch_group(Group *g, const ComputeLaunch &ca) {
@@ -940,23 +990,14 @@ bool launch_group(Group *g, const ComputeLaunch &ca) {
   GroupLaunch a{};
   a.c = c; a.q = ca.q; a.out = ca.out; a.head0 = ca.head0; a.heads_in_call = ca.heads_in_call; a.nq = ca.nq;
   a.n = ca.n; a.status = g->d_status;
-  const int nt = a.nq <= 2 ? 1 : 2; // tensor-core column tiles, two queries each
-  a.groups_per_head = (a.nq + 2 * nt - 1) / (2 * nt);
-  a.per_group = (a.nq + a.groups_per_head - 1) / a.groups_per_head;
-  const long long items = (long long)a.heads_in_call * a.groups_per_head;
-  const long long items_base = (long long)a.heads_in_call * a.nq;
-  // Heads are cut anywhere on 64-token boundaries, so that all groups get equal shares.  They stay
-  // whole where there are more queries than arrival counters (then there are many heads), and where
-  // room for the pieces' partials cannot be had: no memory, or a stream capture under way.
-  bool cut = items_base <= MAX_COUNTED_ITEMS;
-  int grid = g->sm_count;
-  if (cut) {
-    a.unit_tokens = GQ_UNIT;
-    a.units = (a.n + GQ_UNIT - 1) / GQ_UNIT;
-    const long long total = items * a.units;
-    // a run of at least 256 tokens, and of a 16th of a head: one warp merges a head's pieces
-    const long long shortest = std::max<long long>(4, a.units / 16);
-    grid = (int)std::max<long long>(1, std::min<long long>(grid, total / (GQ_GROUPS * shortest)));
+  const GroupCut p = group_cut(g->sm_count, a.heads_in_call, a.nq, a.n);
+  a.groups_per_head = p.groups_per_head;
+  a.per_group = p.per_group;
+  a.unit_tokens = GQ_UNIT;
+  a.units = p.units;
+  int grid = p.grid;
+  bool cut = p.cut;
+  if (cut) { // no room for the pieces' partials (no memory, or a stream capture under way): heads stay whole
     const size_t bytes = group_scratch_bytes(c, grid * GQ_GROUPS, a.per_group); // at most 1.2 MB
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (bytes > g->scratch_bytes && (cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)) cut = false;
@@ -967,17 +1008,18 @@ bool launch_group(Group *g, const ComputeLaunch &ca) {
   if (!cut) {
     a.unit_tokens = a.n;
     a.units = 1;
-    grid = (int)std::max<long long>(1, std::min<long long>(g->sm_count, items / GQ_GROUPS));
+    grid = (int)std::max<long long>(1, std::min<long long>(g->sm_count, p.items / GQ_GROUPS));
   }
-  if (c.padded == 128) return nt == 1 ? launch_group_kv<128, 1>(g, a, grid) : launch_group_kv<128, 2>(g, a, grid);
-  return nt == 1 ? launch_group_kv<64, 1>(g, a, grid) : launch_group_kv<64, 2>(g, a, grid);
+  if (c.padded == 128) return p.nt == 1 ? launch_group_kv<128, 1>(g, a, grid) : launch_group_kv<128, 2>(g, a, grid);
+  return p.nt == 1 ? launch_group_kv<64, 1>(g, a, grid) : launch_group_kv<64, 2>(g, a, grid);
 }
 
 bool launch_general_or_stream(Group *g, ComputeLaunch &a, bool want_partial_out, float *partial_out) {
   const CacheView &c = g->c;
   const int policy = g_policy.load();
   const bool can_stream = !a.use_mirror && stream_supported(c);
-  if (!a.use_mirror && !want_partial_out && policy != 1 && (can_stream || policy == 0) && group_applies(c, a.heads_in_call, a.nq, a.n))
+  if (!a.use_mirror && !want_partial_out && policy != 1 && (can_stream || policy == 0) &&
+      group_applies(c, g->sm_count, can_stream, a.heads_in_call, a.nq, a.n))
     return launch_group(g, a);
   if (can_stream && policy != 1) return launch_stream(g, a, want_partial_out, partial_out);
   if (policy == 2) { set_error("compute: shape not covered by the streaming kernel"); return false; }

@@ -86,3 +86,37 @@ def test_grouped_queries_non_finite(gpu_lib):
     same = torch.ones_like(rest)
     same[0, 1] = same[1] = False
     assert torch.equal(got[same], want[same])
+
+
+def _us(torch, fn, calls=20, batches=5):
+    """Best time of a call, back to back on the device."""
+    fn(), fn(), torch.cuda.synchronize()
+    best = float("inf")
+    for _ in range(batches):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        e[0].record()
+        for _ in range(calls):
+            fn()
+        e[1].record()
+        torch.cuda.synchronize()
+        best = min(best, e[0].elapsed_time(e[1]) / calls * 1e3)
+    return best
+
+
+@pytest.mark.parametrize("heads,n,nq,dim,kb,vb", [(1, 131072, 4, 128, 4, 2), (4, 131072, 2, 128, 2, 2), (8, 131072, 2, 128, 3, 3),
+                                                  (16, 4096, 8, 128, 4, 2), (32, 4096, 7, 128, 2, 4)])
+def test_calls_that_the_streaming_kernel_does_faster_stay_there(gpu_lib, heads, n, nq, dim, kb, vb):
+    """Few heads give compute_group_kernel too few runs to fill the chip, and small calls do not pay for its
+    launch.  compute_partial always walks the streaming kernel over the same rows; the grouped kernel takes
+    1.35 to 4 times as long here, and 25 % is far above what two runs of one kernel differ by."""
+    import torch
+    from adaptq_b200 import MHAContext
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    ctx = MHAContext(heads, dim, kb, vb, n, seed=1, v_mass=0.0, hybrid_thresh=0)
+    for t in range(0, n, 32768):
+        k, v = (torch.randn((min(32768, n - t), heads, dim), device="cuda", generator=gen) for _ in range(2))
+        ctx.append_all(k, v)
+    q = torch.randn((heads, nq, dim), device="cuda", generator=gen)
+    out, part = torch.empty_like(q), ctx.compute_partial(q)
+    chosen, stream = _us(torch, lambda: ctx.compute_all(q, out=out)), _us(torch, lambda: ctx.compute_partial(q, out=part))
+    assert chosen < 1.25 * stream, (chosen, stream)
