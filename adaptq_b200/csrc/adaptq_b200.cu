@@ -1026,12 +1026,31 @@ bool launch_general_or_stream(Group *g, ComputeLaunch &a, bool want_partial_out,
   return launch_general(g, a, want_partial_out, partial_out);
 }
 
-// The FP32 window on its own kernel (whole float4 rows up to 128 columns).
-bool window_applies(const CacheView &c) { return c.dim % 4 == 0 && c.dim <= WK_MAX_DIM; }
+// Blocks that share a (head, query) in window_kernel: 64 tokens each up to a full cluster while the
+// call is smaller than two blocks per SM; beyond that throughput counts, and fewer, longer blocks
+// waste less (128 heads x 32 queries x 300 tokens x 8: one block 159 us, eight 463, the general kernel
+// 230), but not longer than 512 tokens, from where on more blocks in flight win again.
+int window_cluster(int sm_count, long long items, int n) {
+  int cluster = 1;
+  while (cluster < WK_MAX_CLUSTER && cluster * WK_TOKENS < n) cluster *= 2;
+  while (cluster > 1 && items * cluster > 2 * sm_count && n <= 256 * cluster) cluster /= 2;
+  return cluster;
+}
+// The FP32 window on its own kernel: whole float4 rows up to 128 columns, where it is the faster one.
+// The general kernel cuts a window over the whole GPU, so it wins for few pairs with windows of
+// thousands of tokens: measured crossings at 4096 / 8192 / 16384 tokens for dim 32 / 64 / 128 and one to
+// four pairs (1 x 16384 x 64: 37 us against 49 here, 1 x 65536 x 128: 93 against 194; 8 x 16384 x 64: 70
+// against 50), and for thousands of pairs of narrow heads with a handful of tokens (9600 x 8 x 32: 74
+// against 84).  At 16 to 512 tokens it takes 1 to 5 times as long; below that the two are within 2 us.
+bool window_applies(const CacheView &c, long long items, int n) {
+  if (c.dim % 4 != 0 || c.dim > WK_MAX_DIM || items * WK_MAX_CLUSTER > 0x7fffffffll) return false;
+  if (n <= 8 && c.padded <= 32 && items >= 2048) return false;
+  return n <= 128 * std::max(16, c.padded) || items * std::max(20, c.padded) >= 320;
+}
 bool launch_window(Group *g, const ComputeLaunch &a) {
-  int cluster = 1; // 64 tokens a block while the cluster lasts
-  while (cluster < WK_MAX_CLUSTER && cluster * WK_TOKENS < a.n) cluster *= 2;
-  const dim3 grid((unsigned)((long long)a.heads_in_call * a.nq * cluster));
+  const long long items = (long long)a.heads_in_call * a.nq;
+  const int cluster = window_cluster(g->sm_count, items, a.n);
+  const dim3 grid((unsigned)(items * cluster));
   launch_attention_clusters(g, window_kernel, grid, cluster, WK_THREADS, 0, a.c, a.q, a.out, a.head0, a.nq, a.n, a.status);
   ++g_launches;
   CUDA_TRY(launch_status(), "compute (window)");
@@ -1056,7 +1075,8 @@ bool compute_device(Group *g, const float *dq, float *dout, int head0, int heads
   a.use_mirror = (c.hyb > 0 && st.size <= c.hyb && st.mirror == st.size) ? 1 : 0;
   const bool quant = c.k_bits != 16 && c.v_bits != 16;
   if (partial_out) return launch_general_or_stream(g, a, true, dout);
-  if (a.use_mirror && g_policy.load() == 0 && window_applies(c)) return launch_window(g, a);
+  if (a.use_mirror && g_policy.load() == 0 && window_applies(c, (long long)heads_in_call * nq, st.size))
+    return launch_window(g, a);
   if (!a.use_mirror && c.v_mass > 0.f && quant) return launch_sparse(g, a);
   return launch_general_or_stream(g, a, false, nullptr);
 }

@@ -4,9 +4,10 @@
 // Replaces the hybrid branch of upstream AttentionHead::compute (attention/attention.cpp:491-523)
 // for head dimensions of whole float4 up to 128; other dimensions take compute_general.cuh.
 //
-// What bounds it: latency.  The window of a head is at most 512 KB and a call has few heads, so
-// the time is the chain launch, row loads, softmax, combination of the parts.  A cluster of up to
-// eight blocks shares a (head, query), 64 tokens each at 512; a warp takes eight tokens at a time
+// What bounds it: latency.  At the default threshold the window of a head is at most 512 KB, and a
+// call has few heads, so the time is the chain launch, row loads, softmax, combination of the parts
+// (longer windows and large calls: window_applies in adaptq_b200.cu).  A cluster of up to eight
+// blocks shares a (head, query), 64 tokens each at 512; a warp takes eight tokens at a time
 // with their keys and values all in flight (one lane per float4), keeps its own running maximum,
 // sum and accumulator, and the parts are combined through shared memory, first in the block, then
 // over the cluster: no partials in global memory, no arrival counter.  In the general kernel the

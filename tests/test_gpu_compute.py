@@ -383,3 +383,35 @@ def test_window_matches_oracle(gpu_lib, orc, dim, n, hyb, nq):
     cpu.append_many(k, v)
     assert_close(ctx.compute_all(q), cpu.compute_batch(q), "window")
     ctx.synchronize()
+
+
+@pytest.mark.parametrize("heads,n,nq,dim", [(1, 65536, 1, 128), (2, 16384, 1, 64), (1, 8192, 1, 32), (128, 300, 32, 8), (128, 300, 32, 32)])
+def test_window_calls_take_the_faster_kernel(gpu_lib, heads, n, nq, dim):
+    """Few heads with a long FP32 window, and many (head, query) pairs with one that does not fill a cluster:
+    the automatic choice takes no longer than the general kernel (policy 1; the window kernel with a full
+    cluster took 1.2 to 2 times as long), 15 % and half a microsecond allowed for the measurement."""
+    import torch
+    from adaptq_b200 import MHAContext
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    k, v = (torch.randn((n, heads, dim), device="cuda", generator=gen) for _ in range(2))
+    q = torch.randn((heads, nq, dim), device="cuda", generator=gen)
+    ctx = MHAContext(heads, dim, 4, 4, n, seed=1, v_mass=0.0, hybrid_thresh=n)
+    ctx.append_all(k, v)
+    out = [torch.empty_like(q), torch.empty_like(q)]
+    best = [float("inf")] * 2
+    try:
+        for _ in range(5):
+            for policy in (0, 1):
+                gpu_lib.adaptq_set_kernel_policy(policy)
+                e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+                ctx.compute_all(q, out=out[policy])
+                e[0].record()
+                for _ in range(20):
+                    ctx.compute_all(q, out=out[policy])
+                e[1].record()
+                torch.cuda.synchronize()
+                best[policy] = min(best[policy], e[0].elapsed_time(e[1]) / 20 * 1e3)
+    finally:
+        gpu_lib.adaptq_set_kernel_policy(0)
+    assert_close(out[0].cpu().numpy(), out[1].cpu().numpy(), "window against the general kernel")
+    assert best[0] < 1.15 * best[1] + 0.5, best
