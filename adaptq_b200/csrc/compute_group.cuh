@@ -390,6 +390,13 @@ __global__ void __launch_bounds__(GQ_THREADS, 1) compute_group_kernel(const Grou
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(GQ_REGS_PRODUCER));
     if (warp_all >= GQ_GROUPS * GQ_WARPS + GQ_GROUPS || lane != 0) return;
     griddep_wait(); // everything the cache holds is read through this thread's copies
+    // The block must not end, nor a stage be written twice, while a copy is under way: once a wait has
+    // given up nothing more is issued, and this thread leaves when every stage's latest copy has
+    // landed (bounded; a stage that was never filled counts as landed).
+    auto drain = [&]() {
+      for (int s = 0; s < PL::STAGES; ++s)
+        if (!mbar_wait(&full[s], s < stage ? phase : phase ^ 1u)) atomicExch(a.status, 1);
+    };
     for (long long u = u_begin; u < u_end;) {
       const int item = (int)(u / a.units), u0 = (int)(u % a.units);
       const int cnt_u = (int)min((long long)(a.units - u0), u_end - u);
@@ -408,6 +415,7 @@ __global__ void __launch_bounds__(GQ_THREADS, 1) compute_group_kernel(const Grou
           const uint8_t *src = pass == 0 ? kb : pass == 1 ? vsb : vb;
           for (int t = c0; t < c1; t += tn) {
             wait_on(&empty[stage], phase ^ 1u);
+            if (*fail != 0) { drain(); return; }
             const int cnt = min(tn, c1 - t);
             // sizes rounded up to 16 bytes run into the slack behind a head's rows and scales, never past it
             const uint32_t bytes = ((uint32_t)(cnt * rowb) + 15u) & ~15u;
@@ -415,6 +423,7 @@ __global__ void __launch_bounds__(GQ_THREADS, 1) compute_group_kernel(const Grou
             if (!AQ_CHECK(a.status, (size_t)t * rowb + bytes <= (pass == 0 ? c.k_stride : pass == 1 ? (size_t)c.s_stride * 4 : c.v_stride) &&
                                         h >= 0 && h < c.n_heads, 13)) {
               *fail = 1; // consumers stop waiting; the block drains
+              drain();
               return;
             }
             mbar_expect_tx(&full[stage], bytes + sbytes);
@@ -425,6 +434,7 @@ __global__ void __launch_bounds__(GQ_THREADS, 1) compute_group_kernel(const Grou
         }
       }
     }
+    drain();
     return;
   }
 
