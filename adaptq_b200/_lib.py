@@ -46,6 +46,7 @@ SYMBOLS = {
     "adaptq_mha_create_seeded": (C.c_void_p, [C.c_int, C.POINTER(C.c_uint64), C.c_int, C.c_int, C.c_int, C.c_int, C.c_float, C.c_int]),
     "adaptq_mha_append_batch": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int]),
     "adaptq_mha_compute_all": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p]),
+    "adaptq_mha_reserve_queries": (C.c_int, [C.c_void_p, C.c_int]),
     "adaptq_mha_compute_all_static": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p]),
     "adaptq_mha_compute_partial_to_peers": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.POINTER(C.c_void_p),
                                                        C.POINTER(C.c_void_p), C.c_int, C.c_int]),

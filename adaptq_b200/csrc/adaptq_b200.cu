@@ -123,7 +123,7 @@ struct Group {
   // device staging for host-pointer calls, and scratch for partials / sparse V
   void *d_stage = nullptr; size_t stage_bytes = 0;
   void *h_stage = nullptr; size_t h_stage_bytes = 0;
-  void *d_scratch_base = nullptr; // header + scratch, one allocation (nullptr while they lie behind the key scales)
+  void *d_scratch_base = nullptr; // header + scratch, one allocation
   void *d_scratch = nullptr; size_t scratch_bytes = 0;
   int *d_counters = nullptr;
   int *d_status = nullptr;
@@ -253,8 +253,7 @@ constexpr size_t SCRATCH_HEADER = 65536;
 constexpr int MAX_COUNTED_ITEMS = (int)(SCRATCH_HEADER / sizeof(int));
 
 // Caches whose grouped queries may go to compute_group_kernel (dense V, 2- to 4-bit rows of padded
-// dimension 64 or 128) get room for its pieces' partials with the handle, behind the key scales,
-// where that is below a tenth of the cache: a later cudaMalloc costs the first call half a millisecond.
+// dimension 64 or 128), and the room for its pieces' partials.
 bool group_rows(const CacheView &c) { return (c.padded == 64 || c.padded == 128) && c.k_bits <= 4 && c.v_bits <= 4; }
 size_t group_scratch_bytes(const CacheView &c, int runs, int per_group) {
   return (size_t)runs * 2 * per_group * (2 + c.padded) * sizeof(float);
@@ -296,13 +295,10 @@ Group *create_group(const char *fn, const char *bad_args_msg, int n_heads, const
   c.sign_words = (P + 31) / 32;
   c.mirror_stride = (size_t)hyb * 2 * dim;
   const char *what = fn;
-  const size_t scale_bytes = (size_t)c.s_stride * n_heads * 4;
-  size_t room = group_scratch_bytes(c, GQ_GROUPS * g->sm_count, 4);
-  if (!group_rows(c) || v_mass > 0.f || (double)n_heads * capacity * (c.k_row + c.v_row + 8) < 10. * (room + SCRATCH_HEADER)) room = 0;
   bool ok = alloc((void **)&c.k_slab, c.k_stride * n_heads, g, what) &&
             alloc((void **)&c.v_slab, c.v_stride * n_heads, g, what) &&
-            alloc((void **)&c.k_scale, scale_bytes + (room ? SCRATCH_HEADER + room : 0), g, what) &&
-            alloc((void **)&c.v_scale, scale_bytes, g, what) &&
+            alloc((void **)&c.k_scale, (size_t)c.s_stride * n_heads * 4, g, what) &&
+            alloc((void **)&c.v_scale, (size_t)c.s_stride * n_heads * 4, g, what) &&
             alloc((void **)&c.signs, (size_t)c.sign_words * n_heads * 4, g, what) &&
             alloc((void **)&g->d_status, 16, g, what);
   if (ok && hyb > 0) ok = alloc((void **)&c.mirror, c.mirror_stride * n_heads * 4, g, what);
@@ -318,14 +314,7 @@ Group *create_group(const char *fn, const char *bad_args_msg, int n_heads, const
     fill_f32_kernel<<<(int)std::min<size_t>((ns + 255) / 256, 4096), 256>>>(c.k_scale, ns, 1.0f);
     fill_f32_kernel<<<(int)std::min<size_t>((ns + 255) / 256, 4096), 256>>>(c.v_scale, ns, 1.0f);
     g_launches += 2;
-    if (room) { // scale_bytes is a multiple of 128
-      char *base = reinterpret_cast<char *>(c.k_scale) + scale_bytes;
-      e = cudaMemsetAsync(base, 0, SCRATCH_HEADER);
-      g->d_counters = reinterpret_cast<int *>(base);
-      g->d_scratch = base + SCRATCH_HEADER;
-      g->scratch_bytes = room;
-    }
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    e = cudaDeviceSynchronize();
   }
   if (e != cudaSuccess) {
     set_error("%s: CUDA error during set-up: %s", fn, cudaGetErrorString(e));
@@ -1380,6 +1369,18 @@ int adaptq_mha_compute_all(adaptq_mha_t h, const float *queries, int queries_per
     return -1;
   clear_error();
   return compute_all_impl(g, queries, queries_per_head, outs, false, "adaptq_mha_compute_all");
+}
+
+int adaptq_mha_reserve_queries(adaptq_mha_t h, int queries_per_head) {
+  MHA_PROLOGUE("adaptq_mha_reserve_queries", -1)
+  if (queries_per_head < 0) { set_error("adaptq_mha_reserve_queries: negative queries_per_head"); return -1; }
+  clear_error();
+  std::lock_guard<std::mutex> lk(g->mu);
+  DeviceGuard dg(g->device);
+  const CacheView &c = g->c;
+  if (c.v_mass > 0.f || !group_applies(c, g->sm_count, stream_supported(c), c.n_heads, queries_per_head, c.cap)) return 0;
+  const GroupCut p = group_cut(g->sm_count, c.n_heads, queries_per_head, c.cap);
+  return !p.cut || ensure_scratch(g, group_scratch_bytes(c, GQ_GROUPS * g->sm_count, p.per_group)) ? 0 : -1;
 }
 
 // One decode step over all heads: append one token per head, then one query per

@@ -87,6 +87,7 @@ class AdapTQCache(DynamicCache):
                 for l in range(n_layers):  # one engine per layer, seeded 42 ^ layer as upstream's examples do
                     self._ctx.append(MHAContext(self.n_kv_heads, head_dim, self._bits[l][0], self._bits[l][1], adaptq_capacity,
                                                 seed=seed ^ l, v_mass=0.0, hybrid_thresh=0))
+                    self._ctx[-1].reserve_queries(self.n_heads // self.n_kv_heads)
 
     # -- DynamicCache surface -----------------------------------------------------------
     def get_seq_length(self, layer_idx: int = 0) -> int:

@@ -172,6 +172,11 @@ class MHAContext:
             raise RuntimeError(_lib.last_error())
         return ok
 
+    def reserve_queries(self, queries_per_head):
+        """Allocate now what compute_all with that many queries per head would allocate on its first call."""
+        if self._L.adaptq_mha_reserve_queries(self._h, queries_per_head) != 0:
+            raise RuntimeError(_lib.last_error())
+
     def decode_step(self, keys, vals, queries, out=None, pos=0):
         """One decode step for all heads: append keys/vals [n_heads, dim], then attend
         with queries [n_heads, dim].  Same result as append_all + compute_all; with

@@ -74,6 +74,7 @@ class BatchedAdaptQAttention(nn.Module):
         head_seeds = [(seed ^ (i * 0xDEADBEEFCAFE)) & 0xFFFFFFFFFFFFFFFF for i in range(heads)]
         self._ctx = MHAContext(batch * heads, dim, k_bits, v_bits, capacity, seeds=head_seeds * batch,
                                v_mass=v_mass, hybrid_thresh=hybrid_thresh)
+        self._ctx.reserve_queries(q_per_kv)
         self.pos = 0
 
     def _flat(self, t: torch.Tensor, shape) -> torch.Tensor:

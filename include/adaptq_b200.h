@@ -46,6 +46,12 @@ int adaptq_mha_append_batch(adaptq_mha_t mha, const float *keys,
 int adaptq_mha_compute_all(adaptq_mha_t mha, const float *queries,
                            int queries_per_head, float *outs);
 
+/* Optional: allocate now the workspace that adaptq_mha_compute_all with up to
+ * queries_per_head queries per head needs once the cache is full.  Otherwise the
+ * first such call allocates it (about half a millisecond, once).  At most 1.5 MB,
+ * and nothing for handles whose calls need none.  Returns 0, or -1. */
+int adaptq_mha_reserve_queries(adaptq_mha_t mha, int queries_per_head);
+
 /* One decode step for every head: append one token per head, then attend
  * with one query per head.  keys, vals, queries, outs: float [n_heads][dim].
  * Equals adaptq_mha_append_batch(mha, keys, vals, 1, token_pos) followed by

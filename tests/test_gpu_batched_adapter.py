@@ -86,3 +86,38 @@ def test_shape_errors(gpu_lib):
         m(torch.zeros((2, 4, 64), device="cuda"), x, x)
     with pytest.raises(ValueError):
         m.prefill(torch.zeros((2, 3, 2, 32), device="cuda"), torch.zeros((2, 3, 2, 32), device="cuda"))
+
+
+def test_grouped_workspace_comes_with_handles_made_for_several_queries(gpu_lib):
+    """Room for the pieces of grouped queries: not in a plain handle, from the start (and once) in a module
+    with several queries per KV head, with the first call elsewhere."""
+    import ctypes as C
+    import torch
+    from adaptq_b200 import BatchedAdaptQAttention, MHAContext, _lib
+    batch, heads, dim, cap = 64, 8, 128, 1024
+    kw = dict(v_mass=0.0, hybrid_thresh=0)
+
+    def device_bytes(ctx):
+        info = _lib.MhaInfo()
+        assert gpu_lib.adaptq_mha_info(ctx._h, C.byref(info)) == 0
+        return info.device_bytes
+
+    rows = batch * heads * (cap * (64 + 32) + 2 * 128 + 2 * 4 * (cap + 32) + 16) + 16  # rows, slack, scales, signs; status word
+    plain = MHAContext(batch * heads, dim, 4, 2, cap, seed=1, **kw)
+    single = BatchedAdaptQAttention(dim, heads, batch, 4, 2, cap, **kw)
+    grouped = BatchedAdaptQAttention(dim, heads, batch, 4, 2, cap, q_per_kv=4, **kw)
+    assert device_bytes(plain) == device_bytes(single._ctx) == rows
+    reserved = device_bytes(grouped._ctx)
+    assert rows < reserved < rows + 2 * 2**20
+    x = lambda *s: torch.randn(s, device="cuda")  # noqa: E731
+    k, v = x(cap - 1, batch * heads, dim), x(cap - 1, batch * heads, dim)
+    plain.append_all(k, v)
+    grouped._ctx.append_all(k, v)
+    grouped(x(batch, heads * 4, dim), x(batch, heads, dim), x(batch, heads, dim))
+    assert device_bytes(grouped._ctx) == reserved
+    q = x(batch * heads, 4, dim)
+    plain.compute_all(q)
+    assert rows < device_bytes(plain) < rows + 2 * 2**20
+    plain.reserve_queries(8)
+    with pytest.raises(RuntimeError):
+        plain.reserve_queries(-1)
