@@ -802,6 +802,8 @@ __global__ void __launch_bounds__(GQ_THREADS, 1) compute_group_kernel(const Grou
           return a.partial + ((size_t)(2 * (r_first + p) + second) * a.per_group + warp) * (2 + P);
         };
         float *pp = piece(run - r_first);
+        if (!AQ_CHECK(a.status, r_first >= 0 && r_last < n_runs && run >= r_first && run <= r_last && hq >= 0 &&
+                                    hq < a.heads_in_call * a.nq && warp < a.per_group, 14)) continue;
         if (lane == 0) { pp[0] = s_m[warp]; pp[1] = L; }
 #pragma unroll
         for (int e = 0; e < EPL; ++e) pp[2 + EPL * lane + e] = v[e];
