@@ -93,6 +93,7 @@ SYMBOLS = {
     "adaptq_kernel_backend_name": (C.c_char_p, []),
     "adaptq_inject_failure": (C.c_int, [C.c_int, C.c_int]),
     "adaptq_kernel_launches": (C.c_ulonglong, []),
+    "adaptq_last_attention_kernel": (C.c_char_p, []),
     "adaptq_set_kernel_policy": (C.c_int, [C.c_int]),
 }
 

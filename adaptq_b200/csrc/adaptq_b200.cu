@@ -43,6 +43,9 @@ extern "C" const char *adaptq_last_error(void) { return tl_error; }
 static std::atomic<unsigned long long> g_launches{0};
 static std::atomic<int> g_policy{0};
 extern "C" unsigned long long adaptq_kernel_launches(void) { return g_launches.load(); }
+// The kernel family of the calling thread's latest attention launch (for tests).
+static thread_local const char *tl_attention = "";
+extern "C" const char *adaptq_last_attention_kernel(void) { return tl_attention; }
 extern "C" int adaptq_set_kernel_policy(int policy) {
   if (policy < 0 || policy > 2) { set_error("adaptq_set_kernel_policy: policy must be 0, 1 or 2"); return -1; }
   g_policy.store(policy);
@@ -650,6 +653,7 @@ bool launch_general_kernel(Group *g, const ComputeLaunch &a, dim3 grid, size_t s
 
 bool launch_general(Group *g, ComputeLaunch &a, bool want_partial_out, float *partial_out) {
   const CacheView &c = g->c;
+  tl_attention = "general";
   const bool mirror = a.use_mirror != 0;
   const bool k_f32 = mirror || c.k_bits == 16;
   const bool v_f32 = mirror || c.v_bits == 16;
@@ -716,6 +720,7 @@ bool launch_sparse_fused_t(Group *g, const ComputeLaunch &a, const float *w, int
 
 bool launch_sparse(Group *g, ComputeLaunch &a) {
   const CacheView &c = g->c;
+  tl_attention = "sparse";
   const int items = a.heads_in_call * a.nq;
   const int ws = (int)round_up((size_t)a.n, 32);
   const size_t cells = (size_t)items * ws;
@@ -798,6 +803,7 @@ bool launch_stream_v(Group *g, const StreamLaunch &a, int grid) {
 
 bool launch_stream_for_shape(Group *g, const StreamLaunch &a) {
   const CacheView &c = a.c;
+  tl_attention = "stream";
   const long long items = (long long)a.heads_in_call * a.nq * a.n_splits;
   const int grid = (int)std::min<long long>(items, g->sm_count);
   if (c.padded == 128) {
@@ -976,6 +982,7 @@ bool group_applies(const CacheView &c, int sm_count, bool can_stream, long long 
 
 bool launch_group(Group *g, const ComputeLaunch &ca) {
   const CacheView &c = g->c;
+  tl_attention = "group";
   GroupLaunch a{};
   a.c = c; a.q = ca.q; a.out = ca.out; a.head0 = ca.head0; a.heads_in_call = ca.heads_in_call; a.nq = ca.nq;
   a.n = ca.n; a.status = g->d_status;
@@ -1039,6 +1046,7 @@ bool window_applies(const CacheView &c, long long items, int n) {
 bool launch_window(Group *g, const ComputeLaunch &a) {
   const long long items = (long long)a.heads_in_call * a.nq;
   const int cluster = window_cluster(g->sm_count, items, a.n);
+  tl_attention = "window";
   const dim3 grid((unsigned)(items * cluster));
   launch_attention_clusters(g, window_kernel, grid, cluster, WK_THREADS, 0, a.c, a.q, a.out, a.head0, a.nq, a.n, a.status);
   ++g_launches;

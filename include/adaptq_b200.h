@@ -219,6 +219,10 @@ int adaptq_mha_export_head(adaptq_mha_t mha, int head_idx, uint8_t *k_rows,
 /* Number of CUDA kernels this library has launched in this process. */
 unsigned long long adaptq_kernel_launches(void);
 
+/* Test hook: the kernel family of the calling thread's latest attention launch --
+ * "general", "stream", "group", "window" or "sparse" ("" before the first). */
+const char *adaptq_last_attention_kernel(void);
+
 /* Force a code path, for tests: 0 = automatic, 1 = general-purpose kernels
  * only, 2 = refuse shapes the specialised kernels do not cover. */
 int adaptq_set_kernel_policy(int policy);

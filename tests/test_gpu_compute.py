@@ -385,6 +385,56 @@ def test_window_matches_oracle(gpu_lib, orc, dim, n, hyb, nq):
     ctx.synchronize()
 
 
+@pytest.mark.parametrize("where,kind", [("k", "nan"), ("k", "big"), ("k", "negbig"), ("v", "nan"), ("v", "zero"), ("k", "negbig_all")])
+@pytest.mark.parametrize("n", [70, 300, 512])
+def test_window_special_rows_over_several_blocks(gpu_lib, orc, n, where, kind):
+    """test_hybrid_window_sum_guard's rows with the window spread over a cluster of two to eight blocks:
+    the special row sits in the last block's share, or all logits of a head are -inf."""
+    from adaptq_b200 import MHAContext
+    heads, dim = 2, 128
+    rng = np.random.default_rng(n)
+    k, v = make_kv(rng, n, heads, dim)
+    if kind == "negbig_all":
+        k[:, 1] = -3e37
+    else:
+        (k if where == "k" else v)[n - 1, 1] = _special_rows(dim)[kind]
+    q = np.abs(rng.standard_normal((heads, dim))).astype(np.float32) + 4.0  # all of one sign: 1e38 rows overflow in any order
+    ctx = MHAContext(heads, dim, 4, 2, 2048, seed=6, v_mass=0.95, hybrid_thresh=512)
+    cpu = CpuHeads(orc, heads, dim, 4, 2, 2048, 6, 0.95, 512)
+    ctx.append_all(k, v)
+    cpu.append_many(k, v)
+    got, want = ctx.compute_all(q), cpu.compute(q)
+    assert gpu_lib.adaptq_last_attention_kernel() == b"window"
+    assert np.isfinite(want[0]).all()
+    for h in range(heads):
+        _assert_same_or_both_nonfinite(got[h], want[h], f"{kind} in {where}, head {h}")
+    ctx.synchronize()
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+def test_window_steps_see_the_token_just_appended(gpu_lib, orc, dim):
+    """Decode steps inside the window: the window kernel, with its cluster attribute, is launched to start
+    beside the append of the same step.  Sizes cross from one block to two, four and eight."""
+    import torch
+    from adaptq_b200 import MHAContext
+    heads, pre, steps = 3, 60, 12
+    rng = np.random.default_rng(dim)
+    for start in (pre, 122, 250):
+        k, v = make_kv(rng, start + steps, heads, dim)
+        ctx = MHAContext(heads, dim, 4, 2, 2048, seed=6, v_mass=0.95, hybrid_thresh=512)
+        cpu = CpuHeads(orc, heads, dim, 4, 2, 2048, 6, 0.95, 512)
+        ctx.append_all(torch.from_numpy(k[:start]).cuda(), torch.from_numpy(v[:start]).cuda())
+        cpu.append_many(k[:start], v[:start])
+        for t in range(start, start + steps):
+            q = (k[t] * 0.5).astype(np.float32)  # points at the new key
+            kd, vd, qd = (torch.from_numpy(x).cuda() for x in (k[t], v[t], q))
+            out = ctx.decode_step(kd, vd, qd, pos=t)
+            assert gpu_lib.adaptq_last_attention_kernel() == b"window"
+            cpu.append_many(k[t:t + 1], v[t:t + 1])
+            assert_close(out.cpu().numpy(), cpu.compute(q), f"token {t}")
+        ctx.synchronize()
+
+
 @pytest.mark.parametrize("heads,n,nq,dim", [(1, 65536, 1, 128), (2, 16384, 1, 64), (1, 8192, 1, 32), (128, 300, 32, 8), (128, 300, 32, 32)])
 def test_window_calls_take_the_faster_kernel(gpu_lib, heads, n, nq, dim):
     """Few heads with a long FP32 window, and many (head, query) pairs with one that does not fill a cluster:

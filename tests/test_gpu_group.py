@@ -8,55 +8,160 @@ from helpers import CpuHeads, assert_close
 
 pytestmark = pytest.mark.gpu
 
-# dim, k_bits, v_bits, tokens, queries per head, capacity (0: tokens)
+SMS = 148
+CHUNK = {1: 2048, 2: 1536}  # tokens between softmaxes, by column tiles (two queries each)
+
+
+def plan(heads, n, nq):
+    """launch_group's split: (column tiles, tokens of the longest piece of a head that one group walks)."""
+    nt = 1 if nq <= 2 else 2
+    items = heads * -(-nq // (2 * nt))
+    if heads * nq > 16384:  # more queries than arrival counters: whole heads
+        return nt, n
+    units = -(-n // 64)
+    total = items * units
+    runs = 2 * max(1, min(SMS, total // (2 * max(4, units // 16))))
+    longest = 0
+    for r in range(runs):
+        u, end = r * total // runs, (r + 1) * total // runs
+        while u < end:
+            cnt = min(units - u % units, end - u)
+            longest = max(longest, min(n, (u % units + cnt) * 64) - u % units * 64)
+            u += cnt
+    return nt, longest
+
+
+# dim, k_bits, v_bits, tokens, queries per head, capacity (0: tokens), heads (0: just above the size where the
+# kernel is considered), several chunks in one piece of a head
 CASES = [
-    (128, 4, 2, 2, 4, 0),        # two tokens; more queries than arrival counters, so heads stay whole
-    (128, 4, 4, 17, 3, 0),       # one row past a tile of 16
-    (64, 2, 3, 33, 5, 0),        # one past the V stream's 32; two query groups, 3 + 2
-    (128, 3, 3, 64, 2, 0),       # exactly one unit of the split
-    (64, 4, 4, 65, 8, 0),
-    (128, 2, 4, 127, 7, 0),
-    (64, 3, 2, 129, 4, 0),       # one past a stage
-    (128, 4, 3, 1535, 4, 0),     # around the chunk of three and four queries
-    (64, 4, 2, 1537, 6, 0),
-    (128, 2, 2, 2049, 2, 0),     # one past the chunk of two
-    (64, 2, 2, 3001, 4, 0),      # 2-bit keys at 64: not a shape of the streaming kernel
-    (128, 3, 2, 40000, 3, 0),    # few heads, many pieces each
-    (64, 3, 4, 1100, 2, 1024),   # wrapped ring
-    (96, 4, 2, 700, 4, 0),       # padded dimension
+    (128, 4, 2, 2, 4, 0, 0, False),        # two tokens; more queries than arrival counters, so heads stay whole
+    (128, 4, 4, 17, 3, 0, 0, False),       # one row past a tile of 16
+    (64, 2, 3, 33, 5, 0, 0, False),        # one past the V stream's 32; two query groups, 3 + 2
+    (128, 3, 3, 64, 2, 0, 0, False),       # exactly one unit of the split
+    (64, 4, 4, 65, 8, 0, 0, False),
+    (128, 2, 4, 127, 7, 0, 0, False),
+    (64, 3, 2, 129, 4, 0, 0, False),       # one past a stage
+    (128, 4, 3, 1536, 4, 0, 400, False),   # exactly one chunk of three and four queries
+    (64, 4, 2, 1537, 6, 0, 200, True),     # one past it
+    (128, 2, 2, 2049, 2, 0, 400, True),    # one past the chunk of two
+    (64, 2, 2, 3001, 4, 0, 0, False),      # 2-bit keys at 64: not a shape of the streaming kernel
+    (128, 3, 2, 40000, 3, 0, 20, True),    # few heads, many pieces each
+    (64, 3, 4, 1100, 2, 1024, 1300, False),  # wrapped ring
+    (96, 4, 2, 700, 4, 0, 300, False),       # padded dimension
+    (64, 4, 2, 2100, 8, 0, 2100, True),    # whole heads longer than a chunk
 ]
 
 
-@pytest.mark.parametrize("dim,kb,vb,n,nq,cap", CASES)
-def test_grouped_queries(gpu_lib, orc, dim, kb, vb, n, nq, cap):
+def fill(torch, gen, ctx, n, heads, dim):
+    """n tokens of normal values, 0.2 % of the keys ten times larger; returns the rows of heads 0, middle and last."""
+    pick, rows, step = [0, heads // 2, heads - 1], [], max(1, 2**27 // (heads * dim))
+    for t in range(0, n, step):
+        k, v = (torch.randn((min(step, n - t), heads, dim), device="cuda", generator=gen) for _ in range(2))
+        k[torch.rand(k.shape, device="cuda", generator=gen) < 0.002] *= 10
+        ctx.append_all(k, v)
+        rows.append((k[:, pick].cpu().numpy(), v[:, pick].cpu().numpy()))
+    return pick, [np.concatenate(r) for r in zip(*rows)]
+
+
+def general(gpu_lib, ctx, q):
+    try:
+        gpu_lib.adaptq_set_kernel_policy(1)
+        return ctx.compute_all(q)
+    finally:
+        gpu_lib.adaptq_set_kernel_policy(0)
+
+
+@pytest.mark.parametrize("dim,kb,vb,n,nq,cap,heads,chunks", CASES)
+def test_grouped_queries(gpu_lib, orc, dim, kb, vb, n, nq, cap, heads, chunks):
     import torch
     from adaptq_b200 import MHAContext
     padded = 64 if dim == 64 else 128
     live = min(n, cap or n)
     row = padded * (kb + vb) // 8 + 8
-    heads = max(3, int((80e6 if nq == 2 else 40e6) / (nq * live * row)) + 1)  # just above the size where the kernel is chosen
+    heads = heads or max(3, int((80e6 if nq == 2 else 40e6) / (nq * live * row)) + 1)
+    if torch.cuda.get_device_properties(0).multi_processor_count == SMS:
+        nt, longest = plan(heads, live, nq)
+        assert (longest > CHUNK[nt]) == chunks
     gen = torch.Generator(device="cuda").manual_seed(dim + 7 * kb + 11 * vb + n)
-    rnd = lambda *s: torch.randn(s, device="cuda", generator=gen)  # noqa: E731
-    k, v, q = rnd(n, heads, dim), rnd(n, heads, dim), rnd(heads, nq, dim)
-    k[torch.rand(k.shape, device="cuda", generator=gen) < 0.002] *= 10
     seeds = [(42 ^ (i % 5)) for i in range(heads)]
     ctx = MHAContext(heads, dim, kb, vb, cap or n, v_mass=0.0, hybrid_thresh=0, seeds=seeds)
-    ctx.append_all(k, v)
+    pick, (k, v) = fill(torch, gen, ctx, n, heads, dim)
+    q = torch.randn((heads, nq, dim), device="cuda", generator=gen)
     before = gpu_lib.adaptq_kernel_launches()
     out = ctx.compute_all(q)
+    assert gpu_lib.adaptq_last_attention_kernel() == b"group"
     assert gpu_lib.adaptq_kernel_launches() - before == 1, "one launch for all queries"
     assert torch.equal(out, ctx.compute_all(q)), "integer sums: the same bits every time"
     ctx.synchronize()
-    pick = [0, heads // 2, heads - 1]
     cpu = CpuHeads(orc, 3, dim, kb, vb, cap or n, 0, seeds=[seeds[i] for i in pick])
-    cpu.append_many(k[:, pick].cpu().numpy(), v[:, pick].cpu().numpy())
+    cpu.append_many(k, v)
     assert_close(out[pick].cpu().numpy(), cpu.compute_batch(q[pick].cpu().numpy()), "against the oracle")
-    try:
-        gpu_lib.adaptq_set_kernel_policy(1)
-        ref = ctx.compute_all(q)
-    finally:
-        gpu_lib.adaptq_set_kernel_policy(0)
-    assert_close(out.cpu().numpy(), ref.cpu().numpy(), "against the general kernel")
+    assert_close(out.cpu().numpy(), general(gpu_lib, ctx, q).cpu().numpy(), "against the general kernel")
+
+
+@pytest.mark.parametrize("nq", [2, 3])
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("vb", [2, 3, 4])
+@pytest.mark.parametrize("kb", [2, 3, 4])
+def test_every_instantiation_over_several_chunks(gpu_lib, kb, vb, dim, nq):
+    """Pieces longer than a chunk: the running maximum, the rescaled accumulator and stages carried over."""
+    import torch
+    from adaptq_b200 import MHAContext
+    heads, n = 360, 3001
+    if torch.cuda.get_device_properties(0).multi_processor_count == SMS:
+        nt, longest = plan(heads, n, nq)
+        assert longest > CHUNK[nt]
+    gen = torch.Generator(device="cuda").manual_seed(dim + 7 * kb + 11 * vb)
+    ctx = MHAContext(heads, dim, kb, vb, n, seed=5, v_mass=0.0, hybrid_thresh=0)
+    fill(torch, gen, ctx, n, heads, dim)
+    q = torch.randn((heads, nq, dim), device="cuda", generator=gen)
+    out = ctx.compute_all(q)
+    assert gpu_lib.adaptq_last_attention_kernel() == b"group"
+    ctx.synchronize()
+    assert_close(out.cpu().numpy(), general(gpu_lib, ctx, q).cpu().numpy(), "against the general kernel")
+
+
+def test_without_room_for_pieces_heads_stay_whole(gpu_lib):
+    """No memory for the pieces' partials, or a stream capture under way that forbids allocating them."""
+    import torch
+    from adaptq_b200 import MHAContext
+    heads, dim, n, nq = 100, 128, 1700, 4
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    made = lambda: MHAContext(heads, dim, 4, 2, n, seed=5, v_mass=0.0, hybrid_thresh=0)  # noqa: E731
+    k, v = (torch.randn((n, heads, dim), device="cuda", generator=gen) for _ in range(2))
+    q = torch.randn((heads, nq, dim), device="cuda", generator=gen)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        ctx, refused, captured = made(), made(), made()
+        for c in (ctx, refused, captured):
+            c.append_all(k, v)
+        want = ctx.compute_all(q)
+        assert gpu_lib.adaptq_last_attention_kernel() == b"group"
+        ref = general(gpu_lib, ctx, q)
+        gpu_lib.adaptq_inject_failure(1, 1)
+        try:
+            got = refused.compute_all(q)
+        finally:
+            gpu_lib.adaptq_inject_failure(1, 0)
+        assert gpu_lib.adaptq_last_attention_kernel() == b"group" and gpu_lib.adaptq_last_error() == b""
+        again = refused.compute_all(q)  # now there is room
+        refused.synchronize()
+        out = torch.empty_like(q)
+        graph = torch.cuda.CUDAGraph()
+        stream.synchronize()
+        with torch.cuda.graph(graph, stream=stream):
+            captured.compute_all(q, out=out)
+        assert gpu_lib.adaptq_last_attention_kernel() == b"group"
+        graph.replay()
+        first = out.clone()
+        out.zero_()
+        graph.replay()
+    torch.cuda.synchronize()
+    captured.synchronize()
+    assert torch.equal(again, want) and torch.equal(first, got) and torch.equal(out, got)
+    for o in (want, got):
+        assert_close(o.cpu().numpy(), ref.cpu().numpy(), "against the general kernel")
 
 
 def test_grouped_queries_non_finite(gpu_lib):
