@@ -376,6 +376,17 @@ bool ensure_scratch(Group *g, size_t bytes) {
   return true;
 }
 
+// Whether a launch may count on that much scratch: not where it would have to be allocated and there is
+// no memory, or a stream capture is under way.
+bool scratch_at_hand(Group *g, size_t bytes) {
+  if (bytes <= g->scratch_bytes) return true;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+  if (ensure_scratch(g, bytes)) return true;
+  clear_error();
+  return false;
+}
+
 // Bring `bytes` at `src` to the device: device pointers pass through, pinned
 // host memory is copied asynchronously, pageable memory goes through the
 // handle's pinned buffer.  `slot_off` places it inside the staging buffer.
@@ -953,10 +964,13 @@ GroupCut group_cut(int sm_count, long long heads, int nq, int n) {
 // Shapes that the streaming kernel does not have (2-bit keys at 64) come from the general kernel,
 // which loses by 1.4 to 3 times as soon as a fifth of the blocks have work (2 heads x 131072 x 8: 98
 // against 70, 1 x 524288 x 8: 143 against 243).
-bool group_applies(const CacheView &c, int sm_count, bool can_stream, long long heads, int nq, int n) {
+bool group_considered(const CacheView &c, long long heads, int nq, int n) {
   if (nq < 2 || !group_rows(c)) return false;
   const double work = (double)heads * nq * n * (c.k_row + c.v_row + 8);
-  if (work < (nq == 2 ? 80e6 : 40e6)) return false; // packed bytes times queries; below, a launch costs more than it saves
+  return work >= (nq == 2 ? 80e6 : 40e6); // packed bytes times queries; below, a launch costs more than it saves
+}
+bool group_applies(const CacheView &c, int sm_count, bool can_stream, long long heads, int nq, int n) {
+  if (!group_considered(c, heads, nq, n)) return false;
   const GroupCut p = group_cut(sm_count, heads, nq, n);
   if (!can_stream) return 5 * p.grid >= sm_count;
   const int runs = GQ_GROUPS * p.grid;
@@ -993,11 +1007,8 @@ bool launch_group(Group *g, const ComputeLaunch &ca) {
   a.units = p.units;
   int grid = p.grid;
   bool cut = p.cut;
-  if (cut) { // no room for the pieces' partials (no memory, or a stream capture under way): heads stay whole
-    const size_t bytes = group_scratch_bytes(c, grid * GQ_GROUPS, a.per_group); // at most 1.2 MB
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (bytes > g->scratch_bytes && (cudaStreamIsCapturing(g->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone)) cut = false;
-    else if (!ensure_scratch(g, bytes)) { clear_error(); cut = false; }
+  if (cut) { // without room for the pieces' partials (at most 1.2 MB) heads stay whole
+    cut = scratch_at_hand(g, group_scratch_bytes(c, grid * GQ_GROUPS, a.per_group));
     a.partial = static_cast<float *>(g->d_scratch);
     a.counters = g->d_counters;
   }
@@ -1010,12 +1021,27 @@ bool launch_group(Group *g, const ComputeLaunch &ca) {
   return p.nt == 1 ? launch_group_kv<64, 1>(g, a, grid) : launch_group_kv<64, 2>(g, a, grid);
 }
 
+// Scratch for the partials of a call's spans on the streaming kernel (exact) or the general kernel (a
+// bound: two spans per SM at most, or one per item).
+size_t spans_scratch_bytes(const Group *g, long long heads, int nq, int n, bool can_stream) {
+  const long long items = heads * nq;
+  long long parts = 2ll * g->sm_count + items;
+  if (can_stream) {
+    int n_splits, span;
+    plan_spans(n, (int)items, g->sm_count, n_splits, span);
+    parts = n_splits > 1 ? n_splits * items : 0;
+  }
+  return (size_t)parts * partial_floats(g->c) * sizeof(float);
+}
+
 bool launch_general_or_stream(Group *g, ComputeLaunch &a, bool want_partial_out, float *partial_out) {
   const CacheView &c = g->c;
   const int policy = g_policy.load();
   const bool can_stream = !a.use_mirror && stream_supported(c);
   if (!a.use_mirror && !want_partial_out && policy != 1 && (can_stream || policy == 0) &&
-      group_applies(c, g->sm_count, can_stream, a.heads_in_call, a.nq, a.n))
+      group_considered(c, a.heads_in_call, a.nq, a.n) &&
+      (group_applies(c, g->sm_count, can_stream, a.heads_in_call, a.nq, a.n) ||
+       !scratch_at_hand(g, spans_scratch_bytes(g, a.heads_in_call, a.nq, a.n, can_stream)))) // the other kernels cannot do without
     return launch_group(g, a);
   if (can_stream && policy != 1) return launch_stream(g, a, want_partial_out, partial_out);
   if (policy == 2) { set_error("compute: shape not covered by the streaming kernel"); return false; }
@@ -1038,10 +1064,16 @@ int window_cluster(int sm_count, long long items, int n) {
 // four pairs (1 x 16384 x 64: 37 us against 49 here, 1 x 65536 x 128: 93 against 194; 8 x 16384 x 64: 70
 // against 50), and for thousands of pairs of narrow heads with a handful of tokens (9600 x 8 x 32: 74
 // against 84).  At 16 to 512 tokens it takes 1 to 5 times as long; below that the two are within 2 us.
-bool window_applies(const CacheView &c, long long items, int n) {
-  if (c.dim % 4 != 0 || c.dim > WK_MAX_DIM || items * WK_MAX_CLUSTER > 0x7fffffffll) return false;
+// It also takes calls that the general kernel cannot: more heads or queries than its grid holds, or no
+// scratch to be had for the partials of its spans.
+bool window_applies(Group *g, long long heads, int nq, int n) {
+  const CacheView &c = g->c;
+  const long long items = heads * nq;
+  if (c.dim % 4 != 0 || c.dim > WK_MAX_DIM || items * window_cluster(g->sm_count, items, n) > 0x7fffffffll) return false;
+  if (heads > 65535 || nq > 65535) return true;
   if (n <= 8 && c.padded <= 32 && items >= 2048) return false;
-  return n <= 128 * std::max(16, c.padded) || items * std::max(20, c.padded) >= 320;
+  return n <= 128 * std::max(16, c.padded) || items * std::max(20, c.padded) >= 320 ||
+         !scratch_at_hand(g, spans_scratch_bytes(g, heads, nq, n, false));
 }
 bool launch_window(Group *g, const ComputeLaunch &a) {
   const long long items = (long long)a.heads_in_call * a.nq;
@@ -1072,7 +1104,7 @@ bool compute_device(Group *g, const float *dq, float *dout, int head0, int heads
   a.use_mirror = (c.hyb > 0 && st.size <= c.hyb && st.mirror == st.size) ? 1 : 0;
   const bool quant = c.k_bits != 16 && c.v_bits != 16;
   if (partial_out) return launch_general_or_stream(g, a, true, dout);
-  if (a.use_mirror && g_policy.load() == 0 && window_applies(c, (long long)heads_in_call * nq, st.size))
+  if (a.use_mirror && g_policy.load() == 0 && window_applies(g, heads_in_call, nq, st.size))
     return launch_window(g, a);
   if (!a.use_mirror && c.v_mass > 0.f && quant) return launch_sparse(g, a);
   return launch_general_or_stream(g, a, false, nullptr);

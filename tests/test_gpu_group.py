@@ -193,6 +193,45 @@ def test_grouped_queries_non_finite(gpu_lib):
     assert torch.equal(got[same], want[same])
 
 
+@pytest.mark.parametrize("heads,n,nq,dim,kb,hyb,usual", [(1, 131072, 4, 128, 4, 0, b"stream"), (1, 300000, 4, 64, 2, 0, b"general"),
+                                                         (1, 65536, 1, 128, 4, 65536, b"general")])
+def test_calls_whose_faster_kernel_needs_scratch_run_without_it(gpu_lib, heads, n, nq, dim, kb, hyb, usual):
+    """The first call of a handle inside a stream capture, or with no memory to be had: the spans' partials of
+    the streaming and general kernels cannot be allocated, so the grouped or the window kernel takes the call."""
+    import torch
+    from adaptq_b200 import MHAContext
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        handles = [MHAContext(heads, dim, kb, 2, n, seed=5, v_mass=0.0, hybrid_thresh=hyb) for _ in range(3)]
+        for t in range(0, n, 32768):
+            k, v = (torch.randn((min(32768, n - t), heads, dim), device="cuda", generator=gen) for _ in range(2))
+            for c in handles:
+                c.append_all(k, v)
+        q = torch.randn((heads, nq, dim), device="cuda", generator=gen)
+        want = handles[0].compute_all(q)
+        assert gpu_lib.adaptq_last_attention_kernel() == usual
+        gpu_lib.adaptq_inject_failure(1, 1)
+        try:
+            refused = handles[1].compute_all(q)
+        finally:
+            gpu_lib.adaptq_inject_failure(1, 0)
+        without = b"window" if hyb else b"group"
+        assert gpu_lib.adaptq_last_attention_kernel() == without
+        captured = torch.empty_like(q)
+        graph = torch.cuda.CUDAGraph()
+        stream.synchronize()
+        with torch.cuda.graph(graph, stream=stream):
+            handles[2].compute_all(q, out=captured)
+        assert gpu_lib.adaptq_last_attention_kernel() == without
+        graph.replay()
+    torch.cuda.synchronize()
+    for o in (refused, captured):
+        assert_close(o.cpu().numpy(), want.cpu().numpy(), "without scratch")
+    for c in handles:
+        c.synchronize()
+
+
 def _us(torch, fn, calls=20, batches=5):
     """Best time of a call, back to back on the device."""
     fn(), fn(), torch.cuda.synchronize()
