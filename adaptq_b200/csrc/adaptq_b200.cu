@@ -262,6 +262,8 @@ size_t group_scratch_bytes(const CacheView &c, int runs, int per_group) {
   return (size_t)runs * 2 * per_group * (2 + c.padded) * sizeof(float);
 }
 
+bool reserve_spans(Group *g, int nq);
+
 Group *create_group(const char *fn, const char *bad_args_msg, int n_heads, const uint64_t *seeds, int dim,
                     int k_bits, int v_bits, int capacity, float v_mass, int hyb, bool single) {
   if (n_heads <= 0 || dim <= 0 || !valid_bits(k_bits) || !valid_bits(v_bits) || capacity < 0 || hyb < 0) {
@@ -325,6 +327,9 @@ Group *create_group(const char *fn, const char *bad_args_msg, int n_heads, const
     free_group(g);
     return nullptr;
   }
+  // The partials of one query per head on a full cache of 10 MB or more: the first call then allocates
+  // nothing (it does if this fails, and for small caches, of which there may be many).
+  if ((double)n_heads * capacity * (c.k_row + c.v_row + 8) >= 10e6 && !reserve_spans(g, 1)) clear_error();
   return g;
 }
 
@@ -1034,6 +1039,21 @@ size_t spans_scratch_bytes(const Group *g, long long heads, int nq, int n, bool 
   return (size_t)parts * partial_floats(g->c) * sizeof(float);
 }
 
+// Scratch for nq queries per head of a full, dense cache on the kernel that they will go to.
+bool reserve_spans(Group *g, int nq) {
+  const CacheView &c = g->c;
+  if (nq < 1 || c.cap < 1 || c.v_mass > 0.f || !stream_supported(c)) return true;
+  size_t bytes;
+  if (group_applies(c, g->sm_count, true, c.n_heads, nq, c.cap)) {
+    const GroupCut p = group_cut(g->sm_count, c.n_heads, nq, c.cap);
+    bytes = p.cut ? group_scratch_bytes(c, GQ_GROUPS * g->sm_count, p.per_group) : 0;
+  } else {
+    bytes = spans_scratch_bytes(g, c.n_heads, nq, c.cap, true);
+  }
+  if (10. * (double)(bytes + SCRATCH_HEADER) > (double)c.n_heads * c.cap * (c.k_row + c.v_row + 8)) return true;
+  return bytes == 0 || ensure_scratch(g, bytes);
+}
+
 bool launch_general_or_stream(Group *g, ComputeLaunch &a, bool want_partial_out, float *partial_out) {
   const CacheView &c = g->c;
   const int policy = g_policy.load();
@@ -1417,10 +1437,7 @@ int adaptq_mha_reserve_queries(adaptq_mha_t h, int queries_per_head) {
   clear_error();
   std::lock_guard<std::mutex> lk(g->mu);
   DeviceGuard dg(g->device);
-  const CacheView &c = g->c;
-  if (c.v_mass > 0.f || !group_applies(c, g->sm_count, stream_supported(c), c.n_heads, queries_per_head, c.cap)) return 0;
-  const GroupCut p = group_cut(g->sm_count, c.n_heads, queries_per_head, c.cap);
-  return !p.cut || ensure_scratch(g, group_scratch_bytes(c, GQ_GROUPS * g->sm_count, p.per_group)) ? 0 : -1;
+  return reserve_spans(g, queries_per_head) ? 0 : -1;
 }
 
 // One decode step over all heads: append one token per head, then one query per

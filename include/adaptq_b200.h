@@ -47,9 +47,10 @@ int adaptq_mha_compute_all(adaptq_mha_t mha, const float *queries,
                            int queries_per_head, float *outs);
 
 /* Optional: allocate now the workspace that adaptq_mha_compute_all with up to
- * queries_per_head queries per head needs once the cache is full.  Otherwise the
- * first such call allocates it (about half a millisecond, once).  At most 1.5 MB,
- * and nothing for handles whose calls need none.  Returns 0, or -1. */
+ * queries_per_head queries per head needs once the cache is full (for one query per
+ * head it comes with the handle).  Otherwise the first such call allocates it.  Nothing
+ * where it would exceed a tenth of the cache, or where the calls need none.
+ * Returns 0, or -1. */
 int adaptq_mha_reserve_queries(adaptq_mha_t mha, int queries_per_head);
 
 /* One decode step for every head: append one token per head, then attend
