@@ -191,6 +191,14 @@ __device__ __forceinline__ float quad_transpose_sum(float (&v)[STEPS], int wl) {
   }
 }
 
+// A producer whose wait has run out issues nothing more, and leaves when every stage's latest copy has
+// landed (bounded): the block must not end while one is under way.
+__device__ __noinline__ void give_up(int *fail, int *status, uint64_t *full, int n_stages, int stage, uint32_t phase) {
+  *reinterpret_cast<volatile int *>(fail) = 1;
+  atomicCAS(status, 0, 1); // a failed check's code stays
+  for (int s = 0; s < n_stages; ++s) mbar_wait(&full[s], s < stage ? phase : phase ^ 1u);
+}
+
 // KB/VB: bits; KW/VW: 32-bit words per packed row (8 or 16; 6 or 12 for 3-bit keys).
 template <int KB, int KW, int VB, int VW>
 __device__ __forceinline__ void compute_stream_body(const StreamLaunch &a) {
@@ -342,9 +350,9 @@ __device__ __forceinline__ void compute_stream_body(const StreamLaunch &a) {
         const int tn = pass == 0 ? TKN : pass == 1 ? CS_STAGE_BYTES / 4 : TVN;
         const uint8_t *src = pass == 0 ? kb : pass == 1 ? vsb : vb;
         for (int t = t0; t < t1; t += tn) {
-          if (*reinterpret_cast<volatile int *>(s_fail) == 0 && !mbar_wait(&empty[stage], phase ^ 1u)) {
-            *reinterpret_cast<volatile int *>(s_fail) = 1;
-            atomicExch(a.status, 1);
+          if (*reinterpret_cast<volatile int *>(s_fail) != 0 || !mbar_wait(&empty[stage], phase ^ 1u)) {
+            give_up(s_fail, a.status, full, n_stages, stage, phase);
+            return;
           }
           const int cnt = min(tn, t1 - t);
           const uint32_t bytes = ((uint32_t)(cnt * rowb) + 15u) & ~15u;
@@ -353,7 +361,7 @@ __device__ __forceinline__ void compute_stream_body(const StreamLaunch &a) {
           // a copy may run into the 128-byte slack behind a head's rows, never past it
           if (!AQ_CHECK(a.status, (size_t)t * rowb + bytes <= (pass == 0 ? c.k_stride : pass == 1 ? (size_t)c.s_stride * 4 : c.v_stride) &&
                                       h >= 0 && h < c.n_heads, 13)) {
-            *reinterpret_cast<volatile int *>(s_fail) = 1; // consumers stop waiting; the block drains
+            give_up(s_fail, a.status, full, n_stages, stage, phase); // consumers stop waiting; the block drains
             return;
           }
           mbar_expect_tx(&full[stage], bytes + sbytes);
