@@ -262,7 +262,7 @@ size_t group_scratch_bytes(const CacheView &c, int runs, int per_group) {
   return (size_t)runs * 2 * per_group * (2 + c.padded) * sizeof(float);
 }
 
-bool reserve_spans(Group *g, int nq);
+void reserve_with_handle(Group *g);
 
 Group *create_group(const char *fn, const char *bad_args_msg, int n_heads, const uint64_t *seeds, int dim,
                     int k_bits, int v_bits, int capacity, float v_mass, int hyb, bool single) {
@@ -327,9 +327,7 @@ Group *create_group(const char *fn, const char *bad_args_msg, int n_heads, const
     free_group(g);
     return nullptr;
   }
-  // The partials of one query per head on a full cache of 10 MB or more: the first call then allocates
-  // nothing (it does if this fails, and for small caches, of which there may be many).
-  if ((double)n_heads * capacity * (c.k_row + c.v_row + 8) >= 10e6 && !reserve_spans(g, 1)) clear_error();
+  reserve_with_handle(g);
   return g;
 }
 
@@ -1042,16 +1040,24 @@ size_t spans_scratch_bytes(const Group *g, long long heads, int nq, int n, bool 
 // Scratch for nq queries per head of a full, dense cache on the kernel that they will go to.
 bool reserve_spans(Group *g, int nq) {
   const CacheView &c = g->c;
-  if (nq < 1 || c.cap < 1 || c.v_mass > 0.f || !stream_supported(c)) return true;
-  size_t bytes;
-  if (group_applies(c, g->sm_count, true, c.n_heads, nq, c.cap)) {
+  if (nq < 1 || c.cap < 1 || c.v_mass > 0.f || !group_rows(c)) return true;
+  const bool can_stream = stream_supported(c);
+  size_t bytes = 0;
+  if (group_applies(c, g->sm_count, can_stream, c.n_heads, nq, c.cap)) {
     const GroupCut p = group_cut(g->sm_count, c.n_heads, nq, c.cap);
     bytes = p.cut ? group_scratch_bytes(c, GQ_GROUPS * g->sm_count, p.per_group) : 0;
-  } else {
-    bytes = spans_scratch_bytes(g, c.n_heads, nq, c.cap, true);
+  } else if (can_stream || (long long)c.n_heads * nq < 2 * g->sm_count) { // the general kernel cuts no heads beyond that
+    bytes = spans_scratch_bytes(g, c.n_heads, nq, c.cap, can_stream);
   }
   if (10. * (double)(bytes + SCRATCH_HEADER) > (double)c.n_heads * c.cap * (c.k_row + c.v_row + 8)) return true;
   return bytes == 0 || ensure_scratch(g, bytes);
+}
+
+// The partials of one query per head on a full cache of 10 MB or more: the first call then allocates
+// nothing (it does if this fails, and for small caches, of which there may be many).
+void reserve_with_handle(Group *g) {
+  const CacheView &c = g->c;
+  if ((double)c.n_heads * c.cap * (c.k_row + c.v_row + 8) >= 10e6 && !reserve_spans(g, 1)) clear_error();
 }
 
 bool launch_general_or_stream(Group *g, ComputeLaunch &a, bool want_partial_out, float *partial_out) {

@@ -123,13 +123,14 @@ def test_grouped_workspace_comes_with_handles_made_for_several_queries(gpu_lib):
         plain.reserve_queries(-1)
     # one long sequence: spans of one query come with the handle, those of more queries when asked for
     n = 100000
-    long = MHAContext(4, dim, 4, 2, n, seed=1, **kw)
-    long.append_all(x(n, 4, dim), x(n, 4, dim))
-    q = x(4, 4, dim)
-    start = device_bytes(long)
-    long.compute_all(q[:, 0].contiguous())
-    assert device_bytes(long) == start
-    long.reserve_queries(4)
-    start = device_bytes(long)
-    long.compute_all(q)
-    assert device_bytes(long) == start
+    for d, bits in ((dim, 4), (64, 2)):  # 2-bit keys at 64: the general kernel
+        long = MHAContext(4, d, bits, 2, n, seed=1, **kw)
+        long.append_all(x(n, 4, d), x(n, 4, d))
+        q = x(4, 4, d)
+        start = device_bytes(long)
+        long.compute_all(q[:, 0].contiguous())
+        assert device_bytes(long) == start
+        long.reserve_queries(4)
+        start = device_bytes(long)
+        long.compute_all(q)
+        assert device_bytes(long) == start

@@ -193,7 +193,7 @@ def test_grouped_queries_non_finite(gpu_lib):
     assert torch.equal(got[same], want[same])
 
 
-@pytest.mark.parametrize("heads,n,nq,dim,kb,hyb,usual", [(1, 90000, 8, 128, 4, 0, b"stream"), (1, 300000, 4, 64, 2, 0, b"general"),
+@pytest.mark.parametrize("heads,n,nq,dim,kb,hyb,usual", [(1, 90000, 8, 128, 4, 0, b"stream"), (1, 240000, 8, 64, 2, 0, b"general"),
                                                          (1, 65536, 1, 128, 4, 65536, b"general")])
 def test_calls_whose_faster_kernel_needs_scratch_run_without_it(gpu_lib, heads, n, nq, dim, kb, hyb, usual):
     """The first call of a handle inside a stream capture, or with no memory to be had: the spans' partials of
