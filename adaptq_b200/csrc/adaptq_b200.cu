@@ -956,14 +956,14 @@ GroupCut group_cut(int sm_count, long long heads, int nq, int n) {
 }
 
 // Calls with several queries per head that compute_group_kernel takes: where it is expected to be
-// the faster one.  Its time is that of its longest run plus the ends of the segments in it; the
-// streaming kernel's is that of its waves of spans, each walked once per query.  The constants (us)
-// are fitted to 1500 pairs of measurements (1 to 16384 heads, 20 to 524288 tokens, 2 to 8 queries, all
-// widths, both dimensions); of those above the sizes below, the choice is within 6 % of the better
-// kernel but for 8 heads (24.6 us against 20.6 at worst), and within 5 % for 398 calls of other sizes.
-// Examples, streaming / this kernel, K4/V2,
-// dim 128, four queries: 512 heads x 4096 tokens 213 / 113, 32 x 16384 60 / 39, 32 x 4096 20 / 27,
-// 4 x 131072 58 / 107, 1 x 131072 26 / 107 (16 runs a head, so a few long heads leave most SMs idle).
+// the faster one.  Its time is that of its longest run plus the ends of the segments in it (a run that
+// is not cut at heads holds one more); the streaming kernel's is that of its waves of spans, each walked
+// once per query.  The constants (us) are fitted to 5013 pairs of measurements above the sizes below
+// (1 to 16384 heads, 20 to 524288 tokens, 2 to 12 queries, all widths, both dimensions): 44 of them, near
+// the crossing, are put on the kernel that is more than 4 % slower, by 19 % at worst; the packed sizes
+// alone put 500 there, by up to six times.  Examples, streaming / this kernel, K4/V2, dim 128, four
+// queries: 512 heads x 4096 tokens 213 / 113, 32 x 16384 60 / 39, 32 x 4096 20 / 27, 4 x 131072 58 / 107,
+// 1 x 131072 26 / 107 (16 runs a head, so a few long heads leave most SMs idle).
 // Shapes that the streaming kernel does not have (2-bit keys at 64) come from the general kernel,
 // which loses by 1.4 to 3 times as soon as a fifth of the blocks have work (2 heads x 131072 x 8: 98
 // against 70, 1 x 524288 x 8: 143 against 243).
@@ -982,18 +982,18 @@ bool group_applies(const CacheView &c, int sm_count, bool can_stream, long long 
     const long long total = p.items * p.units;
     run = (double)total / runs;
     const bool aligned = total % runs == 0 && ((total / runs) % p.units == 0 || p.units % (total / runs) == 0);
-    segments = aligned ? std::max(1., run / p.units) : std::min(std::max(1., run), run / p.units + 1.);
+    segments = aligned ? std::max(1., run / p.units) : std::min(std::max(1., run), std::ceil(run / p.units) + 1.);
   } else {
     segments = (double)((p.items + runs - 1) / runs);
     run = segments * ((n + GQ_UNIT - 1) / GQ_UNIT);
   }
   const bool two = p.nt == 1, narrow = c.padded == 64;
-  const double here = 9.7 + (two ? 4.5 : 8.7) * segments + (narrow ? (two ? 3.8 : 4.6) : (two ? 7.3 : 10.9)) * run * GQ_UNIT * 1e-3;
+  const double here = 8.4 + (two ? 2.9 : 5.5) * segments + (narrow ? (two ? 5.0 : 5.1) : (two ? 7.0 : 9.2)) * run * GQ_UNIT * 1e-3;
   int n_splits, span;
   plan_spans(n, (int)(heads * nq), sm_count, n_splits, span);
   const long long waves = (heads * nq * n_splits + sm_count - 1) / sm_count;
   const int lookups = c.padded / 4 * ((c.k_bits == 2 ? 1 : 2) + (c.v_bits == 2 ? 1 : 2)); // table reads and bucket adds per token
-  const double stream = 6.8 + (double)waves * (3.6 + 0.026 * lookups * std::min(span, n) * 1e-3);
+  const double stream = 7.8 + (double)waves * (3.0 + 0.024 * lookups * std::min(span, n) * 1e-3);
   return here < stream;
 }
 
