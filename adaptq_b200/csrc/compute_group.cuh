@@ -32,7 +32,7 @@
 // What bounds it (512 heads x 4096 tokens, K4/V2, dim 128, four queries: 110 us, 27 warp
 // instructions per token): the 16 warps that 64 accumulators and 32 operand registers a thread leave
 // room for keep the issue slots half busy; integer pipe 41 %, shared-memory wavefronts 43 %, tensor
-// pipe 28 %.  Of a warp's time the K stream takes 35 %, the V stream 24 %, softmax and weights 17 %,
+// pipe 30 %.  Of a warp's time the K stream takes 35 %, the V stream 24 %, softmax and weights 17 %,
 // the ends of segments 18 %.
 #pragma once
 #include "common.cuh"
